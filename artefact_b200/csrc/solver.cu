@@ -292,6 +292,8 @@ __device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b)
 __device__ __forceinline__ float2 vsub(float2 a, float2 b) { return f2sub(a, b); }
 __device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float2 vmul(float2 a, float2 b) { return f2mul(a, b); }
+__device__ __forceinline__ float vmul_only(float a, float b, float2) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float2 vmul_only(float2 a, float2 b, float2 z) { return f2mul_only(a, b, z); }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return f2fma(a, b, c); }
 __device__ __forceinline__ void vsplat(float &d, float v) { d = v; }
@@ -308,235 +310,399 @@ __device__ __forceinline__ float n1_acc(float n, float2 dx, float2 dy) { return 
 __device__ __forceinline__ float h_acc(float n, float t) { return __fadd_rn(n, t); }
 __device__ __forceinline__ float h_acc(float n, float2 t) { return __fadd_rn(__fadd_rn(n, t.x), t.y); }
 
-// Narrow sweep state of one group of channels (one channel, or a packed pair).
+// sigma_c = step / ||g_c|| from the sums of g^2 of groups of eight norm strips.
+// sigma_trees, by 256 threads: the n groups in fp64 over the threads, then each
+// warp's tree into s_dred. sigma_final, after a barrier, by a thread per
+// channel c: the eight warps in order.
+template <int NCH, class GROUP>
+__device__ __forceinline__ void sigma_trees_of(int n, double (*s_dred)[NCH], GROUP group)
+{
+    const int tid = threadIdx.x;
+    double acc[NCH];
+#pragma unroll
+    for (int c = 0; c < NCH; c++) acc[c] = 0.0;
+#pragma unroll 2
+    for (int b = tid; b < n; b += 256) {
+        float s[NCH];
+        group(b, s);
+#pragma unroll
+        for (int c = 0; c < NCH; c++) acc[c] += (double)s[c];
+    }
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int c = 0; c < NCH; c++) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    }
+    if ((tid & 31) == 0) {
+#pragma unroll
+        for (int c = 0; c < NCH; c++) s_dred[tid >> 5][c] = acc[c];
+    }
+}
+
+template <int NCH>
+__device__ __forceinline__ void sigma_trees(const float4 *groups, int n, double (*s_dred)[NCH])
+{
+    sigma_trees_of<NCH>(n, s_dred, [&](int b, float(&s)[NCH]) {
+        const float4 v = __ldcg(groups + b);
+        const float e[3] = {v.x, v.y, v.z};
+#pragma unroll
+        for (int c = 0; c < NCH; c++) s[c] = e[c];
+    });
+}
+
+template <int NCH>
+__device__ __forceinline__ float sigma_final(const double (*s_dred)[NCH], int c, float step)
+{
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) s += s_dred[w][c];
+    const double nrm = sqrt(s);
+    return nrm > 0.0 ? (float)((double)step / nrm) : 0.f;
+}
+
+// Narrow sweep state of one group of channels (one channel, or a packed pair):
+// the row's y with its left and right neighbours, the differences of the row
+// above, the gradient of the row above (Gm) and of this row (G0) so far, and
+// the terms of the row.
 template <class T>
 struct NarrowGroup {
-    T yv, dxp, dyp, Gm, G0, Gp, ssq, ring[SWEEP_PF_N], pring[SWEEP_PPF_N];
-    T yn, pr, dx, dy, gxx, gyy, gs;
+    T yv, yl, yr, dxp, dyp, Gm, G0, ssq;
+    T yn, ynl, ynr, pr, dx, dy, gxx, gyy, gs;
+    T u, v, w, au, cen, bv;
 };
 
-// Narrow variant of the gradient sweep: the same terms with one column per
-// lane, so more warps cover an image and small images fill the GPU better.
-// One warp per strip of SWEEP_OUT_N output columns and strip_rows rows; lane L
-// holds column xs - 2 + L. Lanes 1..30 form the per-pixel terms, lanes 2..29
-// write g. Rows and columns outside the image are read clamped (replicated
-// edges make the reference's last-row/column forward differences vanish,
-// compute_step_tv.rs:105-120) and their terms are zero, which reproduces the
-// reference's scatter guards. Rows are prefetched two ahead of use. With two
-// or three channels, two of them run as a packed pair (channel 0 alone with
-// three), which halves their arithmetic instructions.
-template <int NCH>
-__global__ void __launch_bounds__(SWEEP_WARPS_N * 32, SWEEP_MIN_BLOCKS_N) k_grad_sweep_n(const ImgDev *__restrict__ imgs,
-                                                                 const int2 *__restrict__ work, float stepmul)
+// State at the start of a walk down rows: y and differences of the row above
+// the first. y0 is the row above that and y1 the row itself, each as left,
+// own and right cell; xin: the lane's column has a right neighbour in the image.
+template <class T>
+__device__ __forceinline__ void narrow_begin(NarrowGroup<T> &g, const T (&y0)[3], const T (&y1)[3], bool xin)
 {
-    __shared__ float s_red[SWEEP_WARPS_N][NCH];
-    __shared__ double s_dred[SWEEP_WARPS_N][NCH];
-    __shared__ int s_last;
-    const unsigned FULL = 0xffffffffu;
+    T zero;
+    vsplat(zero, 0.f);
+    g.yl = y1[0];
+    g.yv = y1[1];
+    g.yr = y1[2];
+    g.dxp = vsel(xin, vsub(y0[2], y0[1]), zero);
+    g.dyp = vsub(y1[1], y0[1]);
+    g.Gm = g.G0 = g.ssq = zero;
+}
+
+// One row of the narrow sweep for all channels: the row's terms, gathered into
+// the accumulators of its own and the two neighbouring output rows; when st()
+// is called, Gm of each group plus its pr is the finished gradient of the row
+// above. ly(c, d) is the next row's y of channel c at this lane's column + d,
+// lp(c) the DCT-distance value of the row above. Cells outside the image hold
+// any finite value: with EDGE, forward differences across the image's last
+// column and row are zero (xin, yin false there; compute_step_tv.rs:105-120),
+// backward ones at the left edge and the top row too (tx0, ty0 false;
+// compute_step_tv2.rs:53-69 -- the neighbour is taken equal to self), and the
+// terms of lanes and rows outside are zero (inside false), which reproduces
+// the reference's scatter guards.
+//
+// The neighbours' y come from the staged rows, not by shuffles: a step's chain
+// then has one round of shuffles instead of three, and loads can be issued
+// ahead. The terms of all channels are formed before their shuffles, so that
+// the shuffles are in flight together.
+template <int NCH, bool EDGE, class LY, class LP, class ST>
+__device__ __forceinline__ void narrow_row(NarrowGroup<float> &A, NarrowGroup<float2> &B, LY ly, LP lp, bool inside,
+                                           bool tx0, bool ty0, bool xin, bool yin, float at, float ag, float2 nz, ST st)
+{
     constexpr bool SOLO = NCH & 1;     // channel 0 alone
     constexpr bool PAIR = NCH >= 2;    // channels P0, P0 + 1 packed
     constexpr int P0 = SOLO ? 1 : 0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (SOLO) {
+        A.ynl = ly(0, -1);
+        A.yn = ly(0, 0);
+        A.ynr = ly(0, 1);
+        A.pr = lp(0);
+    }
+    if constexpr (PAIR) {
+        B.ynl = make_float2(ly(P0, -1), ly(P0 + 1, -1));
+        B.yn = make_float2(ly(P0, 0), ly(P0 + 1, 0));
+        B.ynr = make_float2(ly(P0, 1), ly(P0 + 1, 1));
+        B.pr = make_float2(lp(P0), lp(P0 + 1));
+    }
+    float n1 = 0.f, n2 = 0.f;
+    auto second = [&](auto &G) {
+        auto zero = G.yv, half = G.yv, two = G.yv;
+        vsplat(zero, 0.f);
+        vsplat(half, 0.5f);
+        vsplat(two, 2.f);
+        G.dx = vsub(G.yr, G.yv);
+        G.dy = vsub(G.yn, G.yv);
+        auto dxl = vsub(G.yv, G.yl), dyl = vsub(G.ynl, G.yl), dxu = G.dxp, dyu = G.dyp;
+        if constexpr (EDGE) {
+            G.dx = vsel(xin, G.dx, zero);
+            G.dy = vsel(yin, G.dy, zero);
+            dxl = vsel(tx0, dxl, G.dx);
+            dyl = vsel(tx0 && yin, dyl, G.dy);
+            dxu = vsel(ty0, dxu, G.dx);
+            dyu = vsel(ty0, dyu, G.dy);
+        }
+        n1 = n1_acc(n1, G.dx, G.dy);
+        const auto axx = vsub(G.dx, dxl), ayx = vsub(G.dy, dyl);
+        const auto ayy = vsub(G.dy, dyu), axy = vsub(G.dx, dxu);
+        const auto sv = vmul_only(half, vadd(axy, ayx), nz);
+        n2 = h_acc(n2, vfma(ayy, ayy, vfma(two, vmul(sv, sv), vmul(axx, axx))));
+        G.gxx = axx;
+        G.gyy = ayy;
+        G.gs = sv;
+    };
+    if constexpr (SOLO) second(A);
+    if constexpr (PAIR) second(B);
+    const float inv1 = ((!EDGE || inside) && n1 > 0.f) ? rsqrtf(n1) : 0.f;
+    const float inv2 = ((!EDGE || inside) && n2 > 0.f) ? rsqrtf(n2) : 0.f;
+    const float at1 = __fmul_rn(at, inv1), ag2 = __fmul_rn(ag, inv2);
+    auto third = [&](auto &G) {
+        auto at1v = G.yv, ag2v = G.yv, two = G.yv;
+        vsplat(at1v, at1);
+        vsplat(ag2v, ag2);
+        vsplat(two, 2.f);
+        const auto b = vmul_only(at1v, G.dy, nz);
+        G.u = vmul_only(ag2v, vadd(G.gs, G.gxx), nz);
+        G.v = vmul_only(ag2v, vadd(G.gyy, G.gs), nz);
+        G.w = vmul_only(ag2v, G.gs, nz);
+        // A packed pair rounds a + u and a + b once, as fused multiply-adds of
+        // a = alpha dx / n1; a lone channel rounds a first.
+        auto ab = b;
+        if constexpr (sizeof(G.yv) == sizeof(float2)) {
+            G.au = vfma(at1v, G.dx, G.u);
+            ab = vfma(at1v, G.dx, b);
+        } else {
+            const auto a = vmul(at1v, G.dx);
+            G.au = vadd(a, G.u);
+            ab = vadd(a, b);
+        }
+        // centre term -(a + b) - 2 (u + v - w)
+        G.cen = vfma(two, vsub(vadd(G.u, G.v), G.w), ab);
+        G.bv = vadd(b, G.v);
+    };
+    if constexpr (SOLO) third(A);
+    if constexpr (PAIR) third(B);
+    auto gather = [&](auto &G) {
+        const auto aul = vup(G.au), ur = vdn(G.u), wr = vdn(G.w), wl = vup(G.w);
+        const auto g0 = vadd(vsub(G.G0, G.cen), vadd(aul, ur));
+        G.Gm = vadd(G.Gm, vsub(G.v, wl));  // the row above is complete
+        G.G0 = vsub(G.bv, wr);             // the row below begins
+        G.cen = g0;                        // this row, in Gm from the next step on
+    };
+    if constexpr (SOLO) gather(A);
+    if constexpr (PAIR) gather(B);
+    st();
+    auto rotate = [&](auto &G) {
+        G.Gm = G.cen;
+        G.dxp = G.dx;
+        G.dyp = G.dy;
+        G.yl = G.ynl;
+        G.yv = G.yn;
+        G.yr = G.ynr;
+    };
+    if constexpr (SOLO) rotate(A);
+    if constexpr (PAIR) rotate(B);
+}
+
+// Narrow variant of the gradient sweep: one warp per strip of SWEEP_OUT_N = 28
+// output columns and strip_rows rows; lane L holds column xs - 2 + L. Lanes
+// 1..30 form the per-pixel terms, lanes 2..29 write g. With two or three
+// channels, two of them run as a packed pair (channel 0 alone with three).
+//
+// Each warp stages its rows of y and of the DCT-distance planes in shared
+// memory, four rows at a time, SWEEP_STAGES_N chunks in all, with asynchronous
+// copies. Loading rows straight into registers ahead of use, as before, made
+// the walk wait (a warp has six scoreboards for all its loads, shuffles and
+// special functions, so waiting for a shuffle could mean waiting for the newest
+// global load), and a third of its 215 instructions per row of 32 columns were
+// addresses, clamps and moves; now it issues 196, 92 of them arithmetic, at 65 %
+// of the issue slots, which with the tail below bounds it. Measured per launch,
+// before -> now: 1920x1080 4:4:4 33.9 -> 31.1 us, 2600x1500 4:4:4 55.8 -> 49.1,
+// 4:2:0 52.9 -> 48.5, 200x136 gray 13.8 -> 11.7. Two columns a lane halve the
+// shuffles but leave too few warps, and packing columns instead of channels
+// needs two moves per shifted operand: 55 and 74 us at 1080p. The last block's
+// reduction, which the whole GPU waits for, takes 2.8 us at 1080p with one group
+// of eight strips a block (7 us with four).
+template <int NCH>
+__global__ void __launch_bounds__(SWEEP_WARPS_N * 32, SWEEP_MIN_BLOCKS_N) k_grad_sweep_n(
+    const ImgDev *__restrict__ imgs, const int2 *__restrict__ work, float stepmul)
+{
+    constexpr bool SOLO = NCH & 1, PAIR = NCH >= 2;
+    constexpr int P0 = SOLO ? 1 : 0;
+    constexpr int YROW = SWEEP_OUT_N + 8, PROW = SWEEP_OUT_N, CH = SWEEP_CHUNK, S = SWEEP_STAGES_N;
+    constexpr int YSTAGE = NCH * CH * YROW, STAGE = YSTAGE + NCH * CH * PROW;
+    extern __shared__ float4 s_dyn[];
+    __shared__ double s_dred[8][NCH];
+    __shared__ float4 s_red[SWEEP_WARPS_N];
+    __shared__ int s_last;
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float *sm = reinterpret_cast<float *>(s_dyn) + warp * S * STAGE;
     const int2 wk = work[blockIdx.x];
     const ImgDev &im = imgs[wk.x];
-    const int W = im.W, H = im.H, pitch = im.pitch, R = im.strip_rows;
     const int strip = wk.y * SWEEP_WARPS_N + warp;
-    NarrowGroup<float> A;
-    NarrowGroup<float2> B;
-    vsplat(A.ssq, 0.f);
-    vsplat(B.ssq, 0.f);
-
     if (strip < im.nstrips) {
+        const int W = im.W, H = im.H, pitch = im.pitch, R = im.strip_rows;
         const int sxi = strip % im.strips_x, syi = strip / im.strips_x;
         const int xs = sxi * SWEEP_OUT_N, ys = syi * R;
-        const int gx = xs - 2 + lane;
-        const int cx = min(max(gx, 0), W - 1);
-        const bool colin = gx >= 0 && gx < W;
-        const bool outlane = lane >= 2 && lane < 30 && gx < W;
-        const int cs = (int)im.cstride;
-        const float *yp = im.y + cx;
-        float *gout = im.g + (outlane ? gx : 0);
-        const float at = im.alpha_tv, ag = im.alpha_tgv;
-        // DCT-distance gradient plane of each channel at this lane's column
-        // (offsets from the first channel's plane), prefetched one row ahead.
-        const float *pbase = im.ch[0].P;
-        int pcol[NCH], psh[NCH], ppitch[NCH];
-        bool pon[NCH];
+        const long long cs = im.cstride;
+        const int nchunk = (R + CH - 1) / CH + 1;
+
+        // Chunk i holds y rows ys - 2 + 4 i + k, columns xs - 4 .. xs + 31 (nine
+        // 16-byte pieces a row; zero outside the image),
+        // and from i = 1 on P rows ys + 4 (i - 1) + k, those finished in the
+        // chunk's steps (a vertically subsampled component's row once for each
+        // of its output rows, so that a row of P lies at a fixed place).
+        static_assert(CH == 4 && YROW == 36 && PROW == 28, "lane maps below");
+        const int yk = lane / 9, yc = lane % 9;      // y piece of this lane; row 3's last four pieces go to
+        const int ec = lane >> 2, ep = 5 + (lane & 3);  // lanes 4 c .. 4 c + 3 for channel c
+        const int xa = xs - 4 + 4 * yc, xb = xs - 4 + 4 * ep;
+        const bool ina = xa >= 0 && xa < W, inb = xb >= 0 && xb < W, extra = lane < 4 * NCH;
+        int ra = ys - 2 + yk, rb = ys + 1;  // image rows of the next chunk's pieces
+        const float *ya = im.y + (long long)ra * pitch + xa, *yb = im.y + (extra ? ec : 0) * cs + (long long)rb * pitch + xb;
+        const int pk = lane / 7, pc = lane % 7;      // P piece (four columns; two samples where sh = 2)
+        int rp = ys + pk;
+        const float *pg[NCH];
+        int pinc[NCH], psh[NCH];
+        bool pin[NCH];
 #pragma unroll
         for (int c = 0; c < NCH; c++) {
             const ChanDev &cd = im.ch[c];
-            pon[c] = cd.alpha_p != 0.f;
-            psh[c] = cd.sv - 1;
-            ppitch[c] = cd.ppitch;
-            pcol[c] = (int)(cd.P - pbase) + (outlane ? (gx >> (cd.sh - 1)) : 0);
+            psh[c] = cd.sh - 1;
+            const int px = (xs + 4 * pc) >> psh[c];
+            pin[c] = lane < 28 && px < cd.cw;
+            pg[c] = cd.P + (long long)(rp >> (cd.sv - 1)) * cd.ppitch + px;
+            pinc[c] = (CH >> (cd.sv - 1)) * cd.ppitch;
         }
-        const int Hm1 = H - 1;
-        auto yrow = [&](int row) -> int { return min(max(row, 0), Hm1) * pitch; };
-        auto ly = [&](int c, int off) -> float { return __ldg(yp + c * cs + off); };
-        auto lp = [&](int c, int row) -> float {
-            return pon[c] ? __ldg(pbase + pcol[c] + (row >> psh[c]) * ppitch[c]) : 0.f;
-        };
-        auto ld_y = [&](auto &g, int off) {
-            if constexpr (sizeof(g) == sizeof(float)) g = ly(0, off);
-            else g = make_float2(ly(P0, off), ly(P0 + 1, off));
-        };
-        auto ld_p = [&](auto &g, int row) {
-            if constexpr (sizeof(g) == sizeof(float)) g = lp(0, row);
-            else g = make_float2(lp(P0, row), lp(P0 + 1, row));
-        };
-        // Rows in flight: ring[k] = y row t + 1 + k, pring[k] = DCT-distance
-        // row t - 1 + k at step t.
-        auto init = [&](auto &G) {
-            using T = decltype(G.yv);
-            T y0;
-            ld_y(y0, yrow(ys - 2));
-            ld_y(G.yv, yrow(ys - 1));
+        const unsigned sm0 = (unsigned)__cvta_generic_to_shared(sm);
+        auto copy_chunk = [&](bool with_p, int slot) {
+            const unsigned st = sm0 + slot * (STAGE * 4);
+            const bool va = ina && (unsigned)ra < (unsigned)H;
+            const float *sa = va ? ya : im.y;  // never an address outside the planes, also where nothing is read
 #pragma unroll
-            for (int k = 0; k < SWEEP_PF_N; k++) ld_y(G.ring[k], yrow(ys + k));
-#pragma unroll
-            for (int k = 0; k < SWEEP_PPF_N; k++) ld_p(G.pring[k], min(max(ys - 2 + k, 0), Hm1));
-            G.dxp = vsub(vdn(y0), y0);
-            G.dyp = vsub(G.yv, y0);
-            vsplat(G.Gm, 0.f);
-            vsplat(G.G0, 0.f);
-            vsplat(G.Gp, 0.f);
-        };
-        if constexpr (SOLO) init(A);
-        if constexpr (PAIR) init(B);
-        // The row loop in two forms: EDGE keeps the image-edge rules; a strip
-        // whose lanes and rows all lie inside the image, away from its first
-        // and last rows and columns, runs without them (warp-uniform choice).
-        auto rows = [&](auto edge_tag) {
-        constexpr bool EDGE = decltype(edge_tag)::value;
-#pragma unroll 2
-        for (int t = ys - 1; t <= ys + R; t++) {
-            const int o = min(t + 1 + SWEEP_PF_N, Hm1) * pitch;
-            const int pr1 = min(max(t - 1 + SWEEP_PPF_N, 0), Hm1);
-            auto load = [&](auto &G) {
-                G.yn = G.ring[0];
-#pragma unroll
-                for (int k = 0; k + 1 < SWEEP_PF_N; k++) G.ring[k] = G.ring[k + 1];
-                ld_y(G.ring[SWEEP_PF_N - 1], o);
-                G.pr = G.pring[0];
-#pragma unroll
-                for (int k = 0; k + 1 < SWEEP_PPF_N; k++) G.pring[k] = G.pring[k + 1];
-                ld_p(G.pring[SWEEP_PPF_N - 1], pr1);
-            };
-            if constexpr (SOLO) load(A);
-            if constexpr (PAIR) load(B);
-            const bool inside = !EDGE || (colin && t >= 0 && t < H);
-            float n1 = 0.f, n2 = 0.f;
-            auto first = [&](auto &G) {
-                G.dx = vsub(vdn(G.yv), G.yv);
-                G.dy = vsub(G.yn, G.yv);
-                n1 = n1_acc(n1, G.dx, G.dy);
-            };
-            if constexpr (SOLO) first(A);
-            if constexpr (PAIR) first(B);
-            const bool tx0 = gx > 0, ty0 = t > 0;
-            auto second = [&](auto &G) {
-                using T = decltype(G.yv);
-                // At the left edge and the top row the backward differences are
-                // zero (compute_step_tv2.rs:53-69): take the neighbour equal to self.
-                T dxl = vup(G.dx), dyl = vup(G.dy), dxu = G.dxp, dyu = G.dyp;
-                if constexpr (EDGE) {
-                    dxl = vsel(tx0, dxl, G.dx);
-                    dyl = vsel(tx0, dyl, G.dy);
-                    dxu = vsel(ty0, dxu, G.dx);
-                    dyu = vsel(ty0, dyu, G.dy);
-                }
-                const T axx = vsub(G.dx, dxl), ayx = vsub(G.dy, dyl);
-                const T ayy = vsub(G.dy, dyu), axy = vsub(G.dx, dxu);
-                T half, two;
-                vsplat(half, 0.5f);
-                vsplat(two, 2.f);
-                const T sv = vmul(half, vadd(axy, ayx));
-                n2 = h_acc(n2, vfma(ayy, ayy, vfma(two, vmul(sv, sv), vmul(axx, axx))));
-                G.gxx = axx;
-                G.gyy = ayy;
-                G.gs = sv;
-            };
-            if constexpr (SOLO) second(A);
-            if constexpr (PAIR) second(B);
-            const float inv1 = (inside && n1 > 0.f) ? rsqrtf(n1) : 0.f;
-            const float inv2 = (inside && n2 > 0.f) ? rsqrtf(n2) : 0.f;
-            const float at1 = __fmul_rn(at, inv1), ag2 = __fmul_rn(ag, inv2);
-            auto third = [&](auto &G) {
-                using T = decltype(G.yv);
-                T at1v, ag2v, two;
-                vsplat(at1v, at1);
-                vsplat(ag2v, ag2);
-                vsplat(two, 2.f);
-                const T a = vmul(at1v, G.dx), b = vmul(at1v, G.dy);
-                const T u = vmul(ag2v, vadd(G.gs, G.gxx));
-                const T v = vmul(ag2v, vadd(G.gyy, G.gs));
-                const T w = vmul(ag2v, G.gs);
-                const T au = vadd(a, u);
-                const T aul = vup(au), ur = vdn(u), wr = vdn(w), wl = vup(w);
-                // centre term -(a + b) - 2 (u + v - w), then the neighbours' a + u and u
-                const T cen = vfma(two, vsub(vadd(u, v), w), vadd(a, b));
-                G.G0 = vadd(vsub(G.G0, cen), vadd(aul, ur));
-                G.Gp = vadd(G.Gp, vsub(vadd(b, v), wr));
-                G.Gm = vadd(G.Gm, vsub(v, wl));
-                G.dxp = G.dx;
-                G.dyp = G.dy;
-                G.yv = G.yn;
-            };
-            if constexpr (SOLO) third(A);
-            if constexpr (PAIR) third(B);
-            const int ro = t - 1;
-            if (outlane && ro >= ys && ro < ys + R && ro < H) {
-                const int go = ro * pitch;
-                if constexpr (SOLO) {
-                    const float gv = vadd(A.Gm, A.pr);
-                    gout[go] = gv;
-                    A.ssq = vfma(gv, gv, A.ssq);
-                }
-                if constexpr (PAIR) {
-                    const float2 gv = vadd(B.Gm, B.pr);
-                    gout[P0 * cs + go] = gv.x;
-                    gout[(P0 + 1) * cs + go] = gv.y;
-                    B.ssq = vfma(gv, gv, B.ssq);
-                }
+            for (int c = 0; c < NCH; c++) cp_async16_zfill(st + c * CH * YROW * 4 + 16 * lane, sa + c * cs, va);
+            if (extra) {
+                const bool vb = inb && rb < H;
+                cp_async16_zfill(st + (ec * CH + 3) * YROW * 4 + 16 * ep, vb ? yb : im.y, vb);
             }
-            auto rotate = [&](auto &G) {
-                G.Gm = G.G0;
-                G.G0 = G.Gp;
-                vsplat(G.Gp, 0.f);
-            };
-            if constexpr (SOLO) rotate(A);
-            if constexpr (PAIR) rotate(B);
-        }
+            ya += CH * pitch;
+            yb += CH * pitch;
+            ra += CH;
+            rb += CH;
+            if (with_p) {
+                const unsigned sp = st + YSTAGE * 4 + pk * PROW * 4 + 16 * pc;
+#pragma unroll
+                for (int c = 0; c < NCH; c++) {
+                    if (rp < H && pin[c]) {
+                        if (psh[c] == 0) cp_async16(sp + c * CH * PROW * 4, pg[c]);
+                        else cp_async8(sp + c * CH * PROW * 4 - 8 * pc, pg[c]);
+                    }
+                    pg[c] += pinc[c];
+                }
+                rp += CH;
+            }
         };
-        const bool interior = xs - 2 >= 1 && xs + 29 <= W - 1 && ys - 1 >= 1 && ys + R + 1 + SWEEP_PF_N <= H - 1;
-        if (interior)
-            rows(std::false_type{});
-        else
-            rows(std::true_type{});
-    }
-    float ssq_c[NCH];
-    if constexpr (SOLO) ssq_c[0] = A.ssq;
-    if constexpr (PAIR) {
-        ssq_c[P0] = B.ssq.x;
-        ssq_c[P0 + 1] = B.ssq.y;
-    }
-
-    // Fixed-order reduction: warp tree, then warps in order, then blocks in order.
+        const int gx = xs - 2 + lane;
+        const bool colin = gx >= 0 && gx < W, tx0 = gx > 0, xin = gx < W - 1;
+        const bool outlane = lane >= 2 && lane < 30 && gx < W;
+        const float at = im.alpha_tv, ag = im.alpha_tgv;
+        const float2 nz = make_float2(im.neg_zero, im.neg_zero);
 #pragma unroll
-    for (int c = 0; c < NCH; c++) {
-        float s = ssq_c[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-        if (lane == 0) s_red[warp][c] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+        for (int i = 0; i < S - 1; i++) {
+            copy_chunk(i > 0, i);
+            cp_async_commit();
+        }
+        float *gp[NCH];
+        const float *pl[NCH];
 #pragma unroll
         for (int c = 0; c < NCH; c++) {
-            float s = 0.f;
-            for (int w = 0; w < SWEEP_WARPS_N; w++) s += s_red[w][c];
-            im.partial[wk.y * 4 + c] = s;
+            gp[c] = im.g + c * cs + (long long)(ys - 2) * pitch + (outlane ? gx : 0);  // the row of the first step's output
+            pl[c] = sm + YSTAGE + c * CH * PROW + (max(lane - 2, 0) >> (im.ch[c].sh - 1));
         }
+        const int nout = min(R, H - ys);  // output rows
+        NarrowGroup<float> A;
+        NarrowGroup<float2> B;
+        auto walk = [&](auto edge_tag) {
+            constexpr bool EDGE = decltype(edge_tag)::value;
+            int slot = 0, next = S - 1;  // stages of chunk i and of the next copy
+#pragma unroll 1
+            for (int i = 0; i < nchunk; i++) {
+                cp_async_wait<S - 2>();
+                __syncwarp();
+                const float *yl = sm + slot * STAGE + 2 + lane;
+                const int po = slot * STAGE;
+                if (i == 0) {
+                    if constexpr (SOLO) {
+                        const float v0[3] = {yl[-1], yl[0], yl[1]}, v1[3] = {yl[YROW - 1], yl[YROW], yl[YROW + 1]};
+                        narrow_begin(A, v0, v1, xin);
+                    }
+                    if constexpr (PAIR) {
+                        auto l2 = [&](int o) {
+                            return make_float2(yl[P0 * CH * YROW + o], yl[(P0 + 1) * CH * YROW + o]);
+                        };
+                        const float2 v0[3] = {l2(-1), l2(0), l2(1)}, v1[3] = {l2(YROW - 1), l2(YROW), l2(YROW + 1)};
+                        narrow_begin(B, v0, v1, xin);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < CH; k++) {
+                    if (k < 2 && i == 0) continue;  // the rows the walk begins from
+                    const int t = ys - 3 + CH * i + k, out = CH * (i - 1) + k;  // row of the terms; output row - ys
+                    narrow_row<NCH, EDGE>(
+                        A, B, [&](int c, int d) { return yl[(c * CH + k) * YROW + d]; },
+                        [&](int c) { return pl[c][po + k * PROW]; }, colin && t >= 0 && t < H, tx0, t > 0, xin, t < H - 1,
+                        at, ag, nz, [&]() {
+                            if (outlane && (unsigned)out < (unsigned)nout) {
+                                if constexpr (SOLO) {
+                                    const float gv = vadd(A.Gm, A.pr);
+                                    gp[0][0] = gv;
+                                    A.ssq = vfma(gv, gv, A.ssq);
+                                }
+                                if constexpr (PAIR) {
+                                    const float2 gv = vadd(B.Gm, B.pr);
+                                    gp[P0][0] = gv.x;
+                                    gp[P0 + 1][0] = gv.y;
+                                    B.ssq = vfma(gv, gv, B.ssq);
+                                }
+                            }
+#pragma unroll
+                            for (int c = 0; c < NCH; c++) gp[c] += pitch;
+                        });
+                }
+                __syncwarp();  // every lane has read the chunk before its stage is filled again
+                if (i + S - 1 < nchunk) copy_chunk(true, next);
+                cp_async_commit();
+                next = slot;
+                slot = slot + 1 == S ? 0 : slot + 1;
+            }
+        };
+        if (xs - 2 >= 1 && xs + 29 <= W - 1 && ys - 1 >= 1 && ys + R + 1 <= H - 1)
+            walk(std::false_type{});
+        else
+            walk(std::true_type{});
+
+        // Sums of g^2 of the strip: each column down its rows, then the warp tree.
+        float sums[3] = {0.f, 0.f, 0.f};
+        if constexpr (SOLO) sums[0] = A.ssq;
+        if constexpr (PAIR) {
+            sums[P0] = B.ssq.x;
+            sums[P0 + 1] = B.ssq.y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int c = 0; c < NCH; c++) sums[c] += __shfl_xor_sync(FULL, sums[c], o);
+        }
+        if (lane == 0) s_red[warp] = make_float4(sums[0], sums[1], sums[2], 0.f);
+    } else if (lane == 0) {
+        s_red[warp] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);  // the block's strips are one group
+        for (int w = 0; w < SWEEP_WARPS_N; w++) {
+            t.x += s_red[w].x;
+            t.y += s_red[w].y;
+            t.z += s_red[w].z;
+        }
+        reinterpret_cast<float4 *>(im.partial)[wk.y] = t;
         __threadfence();
         const unsigned done = atomicAdd(im.counter, 1u);
         s_last = done == (unsigned)(im.ncta - 1);
@@ -544,31 +710,10 @@ __global__ void __launch_bounds__(SWEEP_WARPS_N * 32, SWEEP_MIN_BLOCKS_N) k_grad
     __syncthreads();
     if (s_last) {
         __threadfence();
-        double acc[NCH];
-#pragma unroll
-        for (int c = 0; c < NCH; c++) acc[c] = 0.0;
-        for (int t = threadIdx.x; t < im.ncta; t += SWEEP_WARPS_N * 32) {
-#pragma unroll
-            for (int c = 0; c < NCH; c++) acc[c] += (double)__ldcg(im.partial + t * 4 + c);
-        }
-#pragma unroll
-        for (int c = 0; c < NCH; c++) {
-            double s = acc[c];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-            if (lane == 0) s_dred[warp][c] = s;
-        }
+        sigma_trees<NCH>(reinterpret_cast<const float4 *>(im.partial), im.ncta, s_dred);
         __syncthreads();
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int c = 0; c < NCH; c++) {
-                double s = 0.0;
-                for (int w = 0; w < SWEEP_WARPS_N; w++) s += s_dred[w][c];
-                const double nrm = sqrt(s);
-                im.sigma[c] = nrm > 0.0 ? (float)((double)(im.step * stepmul) / nrm) : 0.f;
-            }
-            atomicExch(im.counter, 0u);
-        }
+        if (tid < NCH) im.sigma[tid] = sigma_final<NCH>(s_dred, tid, im.step * stepmul);
+        if (tid == 0) atomicExch(im.counter, 0u);
     }
 }
 
@@ -1608,6 +1753,12 @@ TuneChoice pick_shape(const ArtContext *ctx, const ImageSpec &sp, long long batc
     return t;
 }
 
+template <int NCH>
+constexpr int sweep_smem()
+{
+    return SWEEP_WARPS_N * SWEEP_STAGES_N * NCH * SWEEP_CHUNK * (2 * SWEEP_OUT_N + 8) * (int)sizeof(float);
+}
+
 template <int SH, int SV, int PW = PROJ_WARPS>
 constexpr int proj_smem()
 {
@@ -1657,7 +1808,13 @@ static void launch_project(int pw, int m, int n, const ImgDev *ddesc, const int4
         launch_project_mode<4>(m, n, ddesc, tk, fnext, s);
 }
 
-// Raises the dynamic shared-memory limit of the projection kernels, once per device.
+template <int NCH>
+static cudaError_t set_sweep_smem()
+{
+    return cudaFuncSetAttribute(k_grad_sweep_n<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, sweep_smem<NCH>());
+}
+
+// Raises the dynamic shared-memory limit of the projection and on-chip kernels, once per device.
 int configure_kernels(int device)
 {
     static std::mutex mu;
@@ -1668,6 +1825,9 @@ int configure_kernels(int device)
     cudaError_t e = set_proj_smem<2>();
     if (e == cudaSuccess) e = set_proj_smem<4>();
     if (e == cudaSuccess) e = set_proj_smem<8>();
+    if (e == cudaSuccess) e = set_sweep_smem<1>();
+    if (e == cudaSuccess) e = set_sweep_smem<2>();
+    if (e == cudaSuccess) e = set_sweep_smem<3>();
     if (e != cudaSuccess) return fail(ART_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     done[device] = 1;
     return ART_OK;
@@ -1808,6 +1968,7 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
         d.cstride = cstride;
         // compute_step_tv.rs:130 and compute_step_tv2.rs:88-89, compute_step.rs:47.
         d.alpha_tv = 1.0f / sqrtf((float)sp.nch);
+        d.neg_zero = -0.0f;
         d.alpha_tgv = (sp.weight / sqrtf(2.0f)) / sqrtf((float)sp.nch);
         // mod.rs:45 and :71.
         d.step = (sqrtf((float)((uint64_t)sp.W * sp.H)) / 2.0f) / sqrtf(1.0f + (float)step_its);
@@ -2113,15 +2274,40 @@ static void launch_iteration(ArtContext *ctx, int it, float fnext, float stepmul
     if (ctx->wcount[2][1])
         k_grad_sweep_q<1><<<ctx->wcount[2][1], SWEEP_WARPS_Q * 32, 0, s>>>(ddesc, work + ctx->wstart[2][1], stepmul);
     if (ctx->wcount[0][3])
-        k_grad_sweep_n<3><<<ctx->wcount[0][3], SWEEP_WARPS_N * 32, 0, s>>>(ddesc, work + ctx->wstart[0][3], stepmul);
+        k_grad_sweep_n<3><<<ctx->wcount[0][3], SWEEP_WARPS_N * 32, sweep_smem<3>(), s>>>(ddesc, work + ctx->wstart[0][3], stepmul);
     if (ctx->wcount[0][2])
-        k_grad_sweep_n<2><<<ctx->wcount[0][2], SWEEP_WARPS_N * 32, 0, s>>>(ddesc, work + ctx->wstart[0][2], stepmul);
+        k_grad_sweep_n<2><<<ctx->wcount[0][2], SWEEP_WARPS_N * 32, sweep_smem<2>(), s>>>(ddesc, work + ctx->wstart[0][2], stepmul);
     if (ctx->wcount[0][1])
-        k_grad_sweep_n<1><<<ctx->wcount[0][1], SWEEP_WARPS_N * 32, 0, s>>>(ddesc, work + ctx->wstart[0][1], stepmul);
+        k_grad_sweep_n<1><<<ctx->wcount[0][1], SWEEP_WARPS_N * 32, sweep_smem<1>(), s>>>(ddesc, work + ctx->wstart[0][1], stepmul);
     if (tm) cudaEventRecordWithFlags(ctx->events[3 + 4 * it], s, cudaEventRecordExternal);
     if (tm) cudaEventRecordWithFlags(ctx->events[4 + 4 * it], s, cudaEventRecordExternal);
     launch_projections(ctx, fnext);
     if (tm) cudaEventRecordWithFlags(ctx->events[5 + 4 * it], s, cudaEventRecordExternal);
+}
+
+// {FISTA factor of the next point, step multiplier} of every iteration. Two
+// phases: iterations - tail steps of the solve's own size, then `tail` steps of
+// tail_stepmul times that size with the FISTA sequence restarted (the last
+// step of the first phase forms y = x). Without a tail this is the reference's
+// loop (mod.rs:49-75): y_0 = x_0 (f_0 = 0), and the projection of iteration k
+// forms y_{k+1} with f_{k+1}. With decay > 0 the first phase's steps shrink
+// geometrically: step k of that phase is decay^k times the solve's step (fp32
+// product).
+static std::vector<float2> iteration_schedule(uint32_t iterations, uint32_t tail, float tail_stepmul, float decay)
+{
+    const uint32_t k1 = iterations - tail;
+    const std::vector<float> fs1 = fista_factors(k1), fs2 = fista_factors(tail);
+    std::vector<float2> out(iterations);
+    float mul = 1.0f;
+    for (uint32_t it = 0; it < iterations; it++) {
+        if (it < k1) {
+            out[it] = make_float2(it + 1 < k1 ? fs1[it + 1] : 0.0f, mul);
+            if (decay > 0.0f) mul *= decay;
+        } else {
+            out[it] = make_float2(it - k1 + 1 < tail ? fs2[it - k1 + 1] : 0.0f, tail_stepmul);
+        }
+    }
+    return out;
 }
 
 // Replays (capturing first if the work changed shape) the fixed-count
@@ -2131,6 +2317,7 @@ static int run_iterations(ArtContext *ctx, uint32_t iterations, uint32_t tail = 
 {
     if (iterations == 0) return ART_OK;
     tail = std::min(tail, iterations);
+    const std::vector<float2> sched = iteration_schedule(iterations, tail, tail_stepmul, decay);
     if (ctx->timing) {
         const size_t need = 2 + 4 * (size_t)iterations;
         while (ctx->events.size() < need) {
@@ -2158,27 +2345,10 @@ static int run_iterations(ArtContext *ctx, uint32_t iterations, uint32_t tail = 
             cudaGraphExecDestroy(ctx->exec);
             ctx->exec = nullptr;
         }
-        // Two phases: iterations - tail steps of the solve's own size, then
-        // `tail` steps of tail_stepmul times that size with the FISTA sequence
-        // restarted (the last step of the first phase forms y = x). Without a
-        // tail this is the reference's loop (mod.rs:49-75).
-        const uint32_t k1 = iterations - tail;
-        const std::vector<float> fs1 = fista_factors(k1), fs2 = fista_factors(tail);
         cudaGraph_t graph;
         ART_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         if (ctx->timing) cudaEventRecordWithFlags(ctx->events[0], s, cudaEventRecordExternal);
-        // y_0 = x_0 (f_0 = 0); the projection of iteration k forms y_{k+1} with f_{k+1}.
-        // With decay > 0 the first phase's steps shrink geometrically: step
-        // k of that phase is decay^k times the solve's step (fp32 product).
-        float mul = 1.0f;
-        for (uint32_t it = 0; it < iterations; it++) {
-            if (it < k1) {
-                launch_iteration(ctx, (int)it, it + 1 < k1 ? fs1[it + 1] : 0.0f, mul);
-                if (decay > 0.0f) mul *= decay;
-            } else {
-                launch_iteration(ctx, (int)it, it - k1 + 1 < tail ? fs2[it - k1 + 1] : 0.0f, tail_stepmul);
-            }
-        }
+        for (uint32_t it = 0; it < iterations; it++) launch_iteration(ctx, (int)it, sched[it].x, sched[it].y);
         if (ctx->timing) cudaEventRecordWithFlags(ctx->events[1], s, cudaEventRecordExternal);
         cudaError_t e = cudaStreamEndCapture(s, &graph);
         if (e != cudaSuccess) return fail(ART_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -3269,7 +3439,8 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
         return fail(ART_ERR_INVALID_ARGUMENT, "image too large: three padded planes must stay below 2^31 floats");
     const int R = 32;
     const int strips_x = (int)((W + SWEEP_OUT_N - 1) / SWEEP_OUT_N), strips_y = (int)((H + R - 1) / R);
-    const int nstrips = strips_x * strips_y, ncta = (nstrips + SWEEP_WARPS_N - 1) / SWEEP_WARPS_N;
+    const int nstrips = strips_x * strips_y;
+    const int ncta = (nstrips + SWEEP_WARPS_N - 1) / SWEEP_WARPS_N;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -3324,6 +3495,7 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
     d.y = d.x + nch * cstride;
     d.g = d.y + nch * cstride;
     d.alpha_tv = 1.0f / sqrtf((float)nch);
+    d.neg_zero = -0.0f;
     d.alpha_tgv = (weight / sqrtf(2.0f)) / sqrtf((float)nch);
     d.step = (sqrtf((float)((uint64_t)W * H)) / 2.0f) / sqrtf(1.0f + (float)iterations);
     unsigned char *misc = base + o_misc;
@@ -3380,11 +3552,11 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
     for (uint32_t it = 0; it < iterations; it++) {
         const float fnext = it + 1 < iterations ? next_factor() : 0.0f;
         if (nch == 3)
-            k_grad_sweep_n<3><<<ncta, SWEEP_WARPS_N * 32, 0, s>>>(ddesc, work, 1.0f);
+            k_grad_sweep_n<3><<<ncta, SWEEP_WARPS_N * 32, sweep_smem<3>(), s>>>(ddesc, work, 1.0f);
         else if (nch == 2)
-            k_grad_sweep_n<2><<<ncta, SWEEP_WARPS_N * 32, 0, s>>>(ddesc, work, 1.0f);
+            k_grad_sweep_n<2><<<ncta, SWEEP_WARPS_N * 32, sweep_smem<2>(), s>>>(ddesc, work, 1.0f);
         else
-            k_grad_sweep_n<1><<<ncta, SWEEP_WARPS_N * 32, 0, s>>>(ddesc, work, 1.0f);
+            k_grad_sweep_n<1><<<ncta, SWEEP_WARPS_N * 32, sweep_smem<1>(), s>>>(ddesc, work, 1.0f);
         for (int m = 3; m >= 0; m--) {
             const int n = mode_off[m + 1] - mode_off[m];
             if (n == 0) continue;

@@ -3,11 +3,12 @@
 // One solver iteration of backend/artefact-lib/pipeline_scalar (mod.rs:49-75,
 // compute_step.rs:8-72) runs as two kernels:
 //   k_grad_sweep  one warp walks down a 28-column strip of all channels (32
-//                 lanes with a 2-column halo) of the FISTA point y_k, keeping a
-//                 rolling window in registers: channel-coupled TV (compute_step_tv.rs:29-93)
-//                 and TGV (compute_step_tv2.rs:32-136) gradients written as a
-//                 gather of the reference's scatter (horizontal neighbours by
-//                 warp shuffles), plus the DCT-distance gradient plane the last
+//                 lanes with a 2-column halo) of the FISTA point y_k, staged in
+//                 shared memory, keeping a rolling window in registers:
+//                 channel-coupled TV (compute_step_tv.rs:29-93) and TGV
+//                 (compute_step_tv2.rs:32-136) gradients written as a gather of
+//                 the reference's scatter (the neighbours' terms by warp
+//                 shuffles), plus the DCT-distance gradient plane the last
 //                 projection left (compute_step_prob.rs:5-60); writes g and
 //                 sums g^2 per channel; the last block of an image reduces the
 //                 sums in a fixed order and stores sigma_c = step / ||g_c||.
@@ -49,7 +50,8 @@ struct ImgDev {
     float *x;              // iterate x_k; channel c at x + c * cstride
     float *y;              // FISTA point y_k = x_k + f_k (x_k - x_{k-1})
     float *g;              // gradient planes
-    float alpha_tv, alpha_tgv, step, pad;
+    float alpha_tv, alpha_tgv, step;
+    float neg_zero;        // -0.0f, where a kernel needs one that the compiler does not know (f2mul_only)
     float *sigma;          // [4] per channel step / ||g||
     float *partial;        // [ncta * 4] per-block sums of g^2
     unsigned int *counter; // sweep blocks done in the current iteration
@@ -67,10 +69,10 @@ constexpr int SWEEP_PF = 4;       // wide sweep: y rows loaded ahead of use
 constexpr int SWEEP_PPF = 3;      // wide sweep: DCT-distance rows loaded ahead of use
 constexpr int SWEEP_OUT = 60;     // wide sweep: output columns per warp strip (32 lanes x 2 columns, 2 of halo each side)
 constexpr int SWEEP_WARPS = 4;    // wide sweep: warps (strips) per block
-constexpr int SWEEP_PF_N = 3;     // narrow sweep: y rows loaded ahead of use
-constexpr int SWEEP_PPF_N = 2;    // narrow sweep: DCT-distance rows loaded ahead of use
 constexpr int SWEEP_OUT_N = 28;   // narrow sweep: 32 lanes x 1 column, 2 of halo each side
-constexpr int SWEEP_WARPS_N = 8;  // narrow sweep: warps per block
+constexpr int SWEEP_WARPS_N = 8;  // narrow sweep: warps (strips) per block, the strips of one norm group
+constexpr int SWEEP_CHUNK = 4;    // narrow sweep: rows staged at a time
+constexpr int SWEEP_STAGES_N = 3; // narrow sweep: staged chunks (the one in use and two in flight)
 constexpr int SWEEP_OUT_Q = 120;  // quad sweep: output columns per warp strip (32 lanes x 4 columns, 4 of halo each side)
 constexpr int SWEEP_WARPS_Q = 4;  // quad sweep: warps per block
 constexpr int SWEEP_MIN_BLOCKS_Q = 2;
@@ -198,6 +200,12 @@ __device__ __forceinline__ void idct8x8_regs(float *a)
 __device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// A product that is rounded on its own whatever uses it: the compiler fuses
+// packed products into later packed sums (__fmul2_rn and __fadd2_rn, and
+// mul.rn.f32x2 and add.rn.f32x2 too), differently from one kernel to the next.
+// a b + (-0) is a b, signed zeros included; the -0 comes from memory, since a
+// constant is folded away and the product fused again.
+__device__ __forceinline__ float2 f2mul_only(float2 a, float2 b, float2 neg_zero) { return f2fma(a, b, neg_zero); }
 __device__ __forceinline__ float2 f2sub(float2 a, float2 b)
 {
     unsigned long long ua, ub, r;
@@ -219,11 +227,32 @@ __device__ __forceinline__ void transpose8(float (*T)[9], int r, float *v)
     for (int k = 0; k < 8; k++) v[k] = T[k][r];
 }
 
-// Asynchronous global -> shared copies of 16 bytes (L2 only), and their fence.
+// Asynchronous global -> shared copies (16 bytes: L2 only), and their fences.
+// The destination is a shared-memory address or pointer.
+__device__ __forceinline__ void cp_async16(unsigned smem, const void *gmem)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+    cp_async16((unsigned)__cvta_generic_to_shared(smem), gmem);
+}
+// The same, filling the destination with zeros where `in` is false (nothing is read then).
+__device__ __forceinline__ void cp_async16_zfill(unsigned smem, const void *gmem, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async8(unsigned smem, const void *gmem)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem), "l"(gmem) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait_all()
