@@ -55,6 +55,10 @@ struct ImgDev {
     float *sigma;          // [4] per channel step / ||g||
     float *partial;        // [ncta * 4] per-block sums of g^2
     unsigned int *counter; // sweep blocks done in the current iteration
+    int res_tiles_x, res_tiles, res_rows;  // on-chip solver: tile grid, rows per tile
+    unsigned long long *res_part;  // on-chip solver over several blocks: [2][nch][nstrips] tagged norm partials
+    unsigned long long *res_sigma; // ... [nch] tagged sigma
+    unsigned long long *res_y;     // ... and tagged border pixels, with y's geometry
     ChanDev ch[3];
     float q[3][64];
     float invq2[3][64];
