@@ -1180,12 +1180,28 @@ __global__ void __launch_bounds__(PW * 32) k_project(const ImgDev *__restrict__ 
 #include "resident.cuh"
 namespace art {
 
-// Initial image (coef.rs:24-92 with the single unboxing of
+// Start of a solve, for all channels of all images in one launch: the caller's
+// block raster (jpeg/mod.rs:25, zune-jpeg mcu.rs:219-285) to the coefficient
+// image, rejecting non-integral or out-of-range float coefficients, and, with
+// INIT, the initial image (coef.rs:24-92 with the single unboxing of
 // pipeline_simd_adaptive/coef.rs:69-95): IDCT of c*q per block, nearest
-// upsampling to full resolution, written as x_0 and y_0 (aux.rs:62-63).
-// Same lane layout as k_project.
-__global__ void __launch_bounds__(PROJ_WARPS * 32) k_init(const ImgDev *__restrict__ imgs,
-                                                         const int4 *__restrict__ tasks, int ntasks)
+// upsampling to full resolution, written as x_0 and y_0 (aux.rs:62-63), and a
+// zero DCT-distance gradient (the reference starts from cos = c q,
+// coef.rs:94-104). Tasks and lanes as in k_project: lane r of a group holds row
+// r of its block. It moves 12 bytes a sample; every lane's reads and writes are
+// whole 16-byte pieces, where single floats a row apart made the image's part
+// alone 70 us at 1920x1080 4:2:0, more than an iteration, and one launch a
+// channel for the coefficients 3 us each (0.4 ms for a batch of 48 images).
+__device__ __forceinline__ void store8(float *p, const float (&v)[8])
+{
+    reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+template <bool INIT>
+__global__ void __launch_bounds__(PROJ_WARPS * 32) k_start(const ImgDev *__restrict__ imgs,
+                                                          const int4 *__restrict__ tasks, int ntasks,
+                                                          unsigned int *err)
 {
     __shared__ float s_t[PROJ_WARPS][4][8][9];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1196,53 +1212,72 @@ __global__ void __launch_bounds__(PROJ_WARPS * 32) k_init(const ImgDev *__restri
     const int c = tk.y, by = tk.z, grp = lane >> 3, r = lane & 7;
     const int bx = tk.w + grp;
     const ChanDev &cd = im.ch[c];
-    const bool act = bx < cd.cw / 8;
+    const int bw = cd.cw / 8;
+    const bool act = bx < bw;
     float(*T)[9] = s_t[warp][grp];
-    float a[8], co[8];
-    load_coef_row(cd.coef + (long long)(by * 8 + r) * cd.cpitch + (act ? bx : 0) * 8, co);
+    alignas(16) int16_t co[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) a[u] = co[u] * __ldg(&im.q[c][r * 8 + u]);
-    transpose8(T, r, a);
-    idct8(a);
-    transpose8(T, r, a);
-    idct8(a);
-    if (!act) return;
-    const int sh = cd.sh, sv = cd.sv;
-    const long long base = c * im.cstride;
-    for (int sy = 0; sy < sv; sy++) {
-        const long long o = base + (long long)(by * 8 * sv + r * sv + sy) * im.pitch + bx * 8 * sh;
+    for (int u = 0; u < 8; u++) co[u] = 0;
+    if (act) {
+        const long long i0 = ((long long)by * bw + bx) * 64 + r * 8;
+        const bool wide = (reinterpret_cast<uintptr_t>(cd.src) & 15) == 0;  // the caller's pointer: any alignment
+        if (cd.coef_type == ART_COEF_F32) {
+            const float *p = static_cast<const float *>(cd.src) + i0;
+            float v[8];
+            if (wide) {
+                const float4 lo = reinterpret_cast<const float4 *>(p)[0], hi = reinterpret_cast<const float4 *>(p)[1];
+                v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+            } else {
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            for (int sx = 0; sx < sh; sx++) {
-                im.x[o + u * sh + sx] = a[u];
-                im.y[o + u * sh + sx] = a[u];
+                for (int u = 0; u < 8; u++) v[u] = p[u];
             }
-    }
-}
-
-// Block raster (jpeg/mod.rs:25, zune-jpeg mcu.rs:219-285) -> coefficient
-// image, rejecting non-integral or out-of-range float coefficients.
-__global__ void k_ingest(const void *__restrict__ src, int type, int bw, long long ncoef, int16_t *__restrict__ dst,
-                         int cpitch, unsigned int *err)
-{
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ncoef) return;
-    const long long b = i >> 6;
-    const int j = (int)(i & 63);
-    const int by = (int)(b / bw), bx = (int)(b % bw);
-    int16_t val;
-    if (type == ART_COEF_F32) {
-        const float x = static_cast<const float *>(src)[i];
-        if (!(x == rintf(x)) || x < -32768.f || x > 32767.f) {
-            atomicOr(err, 1u);
-            val = 0;
+            bool bad = false;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const bool ok = v[u] == rintf(v[u]) && v[u] >= -32768.f && v[u] <= 32767.f;
+                bad |= !ok;
+                co[u] = ok ? (int16_t)v[u] : (int16_t)0;
+            }
+            if (bad) atomicOr(err, 1u);
         } else {
-            val = (int16_t)x;
+            const int16_t *p = static_cast<const int16_t *>(cd.src) + i0;
+            if (wide) {
+                *reinterpret_cast<uint4 *>(co) = *reinterpret_cast<const uint4 *>(p);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 8; u++) co[u] = p[u];
+            }
         }
-    } else {
-        val = static_cast<const int16_t *>(src)[i];
+        int16_t *dst = const_cast<int16_t *>(cd.coef) + (long long)(by * 8 + r) * cd.cpitch + bx * 8;
+        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(co);
     }
-    dst[(long long)(by * 8 + (j >> 3)) * cpitch + bx * 8 + (j & 7)] = val;
+    if constexpr (INIT) {
+        float a[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) a[u] = (float)co[u] * __ldg(&im.q[c][r * 8 + u]);
+        transpose8(T, r, a);
+        idct8(a);
+        transpose8(T, r, a);
+        idct8(a);
+        if (!act) return;
+        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        store8(cd.P + (long long)(by * 8 + r) * cd.ppitch + bx * 8, zero);
+        const int sh = cd.sh, sv = cd.sv;
+        for (int sy = 0; sy < sv; sy++) {
+            const long long o = c * im.cstride + (long long)((by * 8 + r) * sv + sy) * im.pitch + bx * 8 * sh;
+            if (sh == 1) {
+                store8(im.x + o, a);
+                store8(im.y + o, a);
+            } else {
+                const float lo[8] = {a[0], a[0], a[1], a[1], a[2], a[2], a[3], a[3]};
+                const float hi[8] = {a[4], a[4], a[5], a[5], a[6], a[6], a[7], a[7]};
+                store8(im.x + o, lo);
+                store8(im.x + o + 8, hi);
+                store8(im.y + o, lo);
+                store8(im.y + o + 8, hi);
+            }
+        }
+    }
 }
 
 // One step of the scalar pipeline's initialisation (coef.rs:29-50): block i
@@ -2085,6 +2120,8 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
             cd.ppitch = (int)align_up(cd.cw, 32);
             // compute_step.rs:20-31: alpha = pweight * 2 * 255 * sqrt(2).
             cd.alpha_p = sp.pweight[c] * 2.0f * 255.0f * sqrtf(2.0f);
+            cd.coef_type = (int)sp.ch[c].coef_type;
+            cd.src = sp.src[c];
             o_coef[i][c] = coef_bytes;
             coef_bytes += align_up((size_t)cd.cpitch * cd.chh * sizeof(int16_t), 256);
             o_p[i][c] = p_floats;
@@ -2175,17 +2212,15 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
     const int ntasks = (int)ctx->h_tasks.size();
     ART_CUDA(cudaMemcpyAsync(ctx->desc.p, ctx->h_desc.data(), nimg * sizeof(ImgDev), cudaMemcpyHostToDevice, s));
     ART_CUDA(cudaMemsetAsync(ctx->misc.p, 0, misc_bytes, s));
-    // The first DCT-distance gradient is zero: the reference starts from cos = c q (coef.rs:94-104).
-    ART_CUDA(cudaMemsetAsync(ctx->pbuf.p, 0, p_floats * sizeof(float), s));
     const ImgDev *ddesc = static_cast<const ImgDev *>(ctx->desc.p);
-    for (int i = 0; i < nimg; i++) {
-        const ImageSpec &sp = specs[i];
-        for (uint32_t c = 0; c < sp.nch; c++) {
-            const long long ncoef = (long long)sp.ch[c].block_w * sp.ch[c].block_h * 64;
-            k_ingest<<<(int)((ncoef + 255) / 256), 256, 0, s>>>(
-                sp.src[c], (int)sp.ch[c].coef_type, (int)sp.ch[c].block_w, ncoef,
-                const_cast<int16_t *>(ctx->h_desc[i].ch[c].coef), ctx->h_desc[i].ch[c].cpitch, ctx->errflag);
-        }
+    const int4 *dtasks = static_cast<const int4 *>(ctx->tasks.p);
+    const int start_grid = (ntasks + PROJ_WARPS - 1) / PROJ_WARPS;
+    if (init_mode == ART_INIT_DECODED) {
+        k_start<true><<<start_grid, PROJ_WARPS * 32, 0, s>>>(ddesc, dtasks, ntasks, ctx->errflag);
+    } else {
+        k_start<false><<<start_grid, PROJ_WARPS * 32, 0, s>>>(ddesc, dtasks, ntasks, ctx->errflag);
+        // The first DCT-distance gradient is zero: the reference starts from cos = c q (coef.rs:94-104).
+        ART_CUDA(cudaMemsetAsync(ctx->pbuf.p, 0, p_floats * sizeof(float), s));
     }
     if (init_mode == ART_INIT_SCALAR_COMPAT) {
         size_t need = 0;
@@ -2360,9 +2395,6 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
             ctx->init_seen = key;
         }
         ctx->net_used = true;
-    } else {
-        k_init<<<(ntasks + PROJ_WARPS - 1) / PROJ_WARPS, PROJ_WARPS * 32, 0, s>>>(
-            ddesc, static_cast<const int4 *>(ctx->tasks.p), ntasks);
     }
     ART_CUDA(cudaGetLastError());
     return ART_OK;
@@ -3705,6 +3737,8 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
         cd.coef = reinterpret_cast<const int16_t *>(base + o_coef[c]);
         cd.P = reinterpret_cast<float *>(base + o_p[c]);
         cd.alpha_p = pweight[c] * 2.0f * 255.0f * sqrtf(2.0f);
+        cd.coef_type = (int)coefs[c].coef_type;
+        cd.src = coefs[c].dct_coefs;
         for (int j = 0; j < 64; j++) {
             const float q = coefs[c].quant_table[j];
             d.q[c][j] = q;
@@ -3715,20 +3749,11 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
     int2 *work = reinterpret_cast<int2 *>(base + o_work);
     int4 *tasks = reinterpret_cast<int4 *>(base + o_tasks);
 
-    // Clear what must start at zero: the norm partials, counter and error flag,
-    // and the first DCT-distance gradient planes.
+    // Clear what must start at zero: the norm partials, counter and error flag.
     NOALLOC_CUDA(cudaMemsetAsync(misc, 0, o_desc - o_misc, s));
-    for (uint32_t c = 0; c < nch; c++)
-        NOALLOC_CUDA(cudaMemsetAsync(d.ch[c].P, 0, (size_t)ppitch[c] * coefs[c].rounded_px_h * sizeof(float), s));
     const int nset = std::max(ncta, ntasks);
     k_noalloc_setup<<<(nset + 255) / 256, 256, 0, s>>>(d, ddesc, work, ncta, tasks, ntasks, plan);
-    for (uint32_t c = 0; c < nch; c++) {
-        const long long ncoef = (long long)coefs[c].block_w * coefs[c].block_h * 64;
-        k_ingest<<<(int)((ncoef + 255) / 256), 256, 0, s>>>(coefs[c].dct_coefs, (int)coefs[c].coef_type,
-                                                             (int)coefs[c].block_w, ncoef,
-                                                             const_cast<int16_t *>(d.ch[c].coef), cpitch[c], errflag);
-    }
-    k_init<<<(ntasks + PROJ_WARPS - 1) / PROJ_WARPS, PROJ_WARPS * 32, 0, s>>>(ddesc, tasks, ntasks);
+    k_start<true><<<(ntasks + PROJ_WARPS - 1) / PROJ_WARPS, PROJ_WARPS * 32, 0, s>>>(ddesc, tasks, ntasks, errflag);
     // FISTA factors as fista_factors() forms them, one step ahead (no host buffer).
     float term = 1.0f;
     auto next_factor = [&term]() {

@@ -38,7 +38,8 @@ struct ChanDev {
     const int16_t *coef;  // coefficient image: coef(8by+v, 8bx+u) = block (bx,by), index v*8+u
     float *P;             // alpha_p * IDCT((cos - c q) / q^2) at component resolution
     float alpha_p;        // pweight * 2 * 255 * sqrt(2); 0 disables the DCT-distance term
-    float pad1;
+    int coef_type;        // ART_COEF_F32 or ART_COEF_I16
+    const void *src;      // the caller's coefficients: blocks in raster order, 64 values each
 };
 
 struct ImgDev {
