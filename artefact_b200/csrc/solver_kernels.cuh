@@ -266,4 +266,12 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Programmatic dependent launch: a kernel launched as a dependent may start
+// when every block of the one before it has called pdl_release or ended, and
+// pdl_wait holds it until that one is complete and its writes are visible. Both
+// do nothing in an ordinary launch. A kernel releases only after its own wait,
+// so a dependent also starts after everything before its predecessor.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 }  // namespace art
