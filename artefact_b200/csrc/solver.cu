@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(SWEEP_WARPS_N * 32, SWEEP_MIN_BLOCKS_N) k_grad
             pg[c] = cd.P + (long long)(rp >> (cd.sv - 1)) * cd.ppitch + px;
             pinc[c] = (CH >> (cd.sv - 1)) * cd.ppitch;
         }
+        const unsigned long long policy = l2_policy(im.l2_fit);  // of P, which is not read again
         pdl_wait();  // from here on it reads what the projections wrote
         pdl_release();
         const unsigned sm0 = (unsigned)__cvta_generic_to_shared(sm);
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(SWEEP_WARPS_N * 32, SWEEP_MIN_BLOCKS_N) k_grad
 #pragma unroll
                 for (int c = 0; c < NCH; c++) {
                     if (rp < H && pin[c]) {
-                        if (psh[c] == 0) cp_async16(sp + c * CH * PROW * 4, pg[c]);
+                        if (psh[c] == 0) cp_async16_l2(sp + c * CH * PROW * 4, pg[c], policy);
                         else cp_async8(sp + c * CH * PROW * 4 - 8 * pc, pg[c]);
                     }
                     pg[c] += pinc[c];
@@ -997,13 +998,17 @@ __global__ void __launch_bounds__(SWEEP_WARPS_Q * 32, SWEEP_MIN_BLOCKS_Q) k_grad
     }
 }
 
+// Warps of the projection blocks that are resident while the gradient sweep ends.
+constexpr int EARLY_WARPS = 148 * 32;
+
 // Descent step and projection of coefficient blocks (compute_step.rs:60-71,
 // compute_projection.rs:8-122), the next FISTA point, and the next
 // DCT-distance gradient (compute_step_prob.rs:20-57) from the clamped
 // coefficients the reference keeps as cos (compute_projection.rs:82).
 // One warp per task {image, channel, block row, first block} covering four
 // blocks. The warp's region of y and g (8 SV rows x 32 SH columns) is staged
-// into shared memory with asynchronous 16-byte copies, one round trip; once g
+// into shared memory with asynchronous 16-byte copies, in one of two orders (FIT:
+// the planes nearly fit L2, l2_fits); once g
 // is consumed (x' = y - sigma g), the same plane receives the region of x,
 // again asynchronously, while the block transforms run. Lane group
 // g = lane / 8 takes block first + g and lane j = lane % 8 its component
@@ -1032,7 +1037,7 @@ __device__ __forceinline__ void load_lane(const float *p, float (&v)[SH])
     }
 }
 
-template <int SH, int SV, int PW = PROJ_WARPS>
+template <int SH, int SV, int PW, bool FIT>
 __global__ void __launch_bounds__(PW * 32) k_project(const ImgDev *__restrict__ imgs,
                                                     const int4 *__restrict__ tasks, int ntasks, float fnext)
 {
@@ -1060,24 +1065,48 @@ __global__ void __launch_bounds__(PW * 32) k_project(const ImgDev *__restrict__ 
     const int pitch = im.pitch;
     float *xw = im.x + c * cs, *yw = im.y + c * cs;
     const float *gb = im.g + c * cs;
-    // Stage the region of y: rows of NC floats, 16-byte chunks; chunks of blocks
-    // past the end of the block row are skipped. Nothing so far depends on the
-    // gradient sweep, so in a dependent launch it overlaps the sweep's tail
-    // (its last blocks, and the last block's reduction alone on the GPU).
+    // Stage the regions of y and g: rows of NC floats, 16-byte chunks; chunks of
+    // blocks past the end of the block row are skipped.
     const int ncol = min(NC, (bw - tk.w) * 8 * SH);  // valid columns, a multiple of 8
     const long long r0 = (long long)(by * 8 * SV) * pitch + tk.w * 8 * SH;
     constexpr int CPR = NC / 4;  // 16-byte chunks per row
-    auto stage = [&](float *dst, const float *src) {
-#pragma unroll
+    auto stage = [&](auto copy) {
         for (int i = lane; i < NR * CPR; i += 32) {
             const int row = i / CPR, ch = i - row * CPR;
-            if (ch * 4 < ncol) cp_async16(dst + row * RS + ch * 4, src + r0 + (long long)row * pitch + ch * 4);
+            if (ch * 4 < ncol) copy(row * RS + ch * 4, r0 + (long long)row * pitch + ch * 4);
         }
     };
-    stage(sy_, yw);
-    // Meanwhile: coefficient row j of this lane's block and its quantisation steps.
+    const unsigned long long policy = FIT ? l2_policy(true) : 0ull;
+    const uint4 *cp = reinterpret_cast<const uint4 *>(cd.coef + (by * 8 + j) * cd.cpitch + (act ? bx : 0) * 8);
+    uint4 raw = make_uint4(0, 0, 0, 0);
+    float sg;
+    if constexpr (FIT) {
+        // y does not depend on the gradient sweep, nor do the coefficients (row j
+        // of this lane's block): in a dependent launch their reads overlap the
+        // sweep's tail, its last blocks and the last block's reduction alone on the
+        // GPU. Blocks that do not start early read the coefficients behind g. g
+        // does not wait for sigma: for a zero step it is staged and not used.
+        stage([&](int so, long long go) { cp_async16(sy_ + so, yw + go); });
+        const bool early = blockIdx.x < EARLY_WARPS / PW;
+        if (early) raw = *cp;
+        pdl_wait();
+        pdl_release();
+        stage([&](int so, long long go) { cp_async16_l2(sg_ + so, gb + go, policy); });
+        sg = __ldcg(im.sigma + c);
+        if (!early) raw = *cp;
+    } else {
+        // Bound by memory throughout: y and g row by row, the coefficients last.
+        pdl_wait();
+        pdl_release();
+        sg = im.sigma[c];
+        const bool stepped = sg != 0.f;
+        stage([&](int so, long long go) {
+            cp_async16(sy_ + so, yw + go);
+            if (stepped) cp_async16(sg_ + so, gb + go);
+        });
+        raw = *cp;
+    }
     float co[8], qv[8], iq[8];
-    load_coef_row(cd.coef + (by * 8 + j) * cd.cpitch + (act ? bx : 0) * 8, co);
 #pragma unroll
     for (int u = 0; u < 8; u++) {
         qv[u] = __ldg(&im.q[c][j * 8 + u]);
@@ -1086,14 +1115,14 @@ __global__ void __launch_bounds__(PW * 32) k_project(const ImgDev *__restrict__ 
     const float ap = cd.alpha_p;  // warp-uniform
     float(*T0)[9] = s_t[warp][0][grp];
     float(*T1)[9] = s_t[warp][1][grp];
-    pdl_wait();
-    pdl_release();
+    // The conversions stay below: above they would hold g back until the
+    // coefficients are here.
+    if constexpr (FIT) asm volatile("" : "+r"(raw.x), "+r"(raw.y), "+r"(raw.z), "+r"(raw.w));
+    convert_coef_row(raw, co);
     // A zero step (sigma = 0: the projection of a start image, or a gradient
-    // of norm zero) leaves x' = y: g is then neither staged nor read, so the
-    // projection of a start needs no zeroed g plane.
-    const float sg = __ldcg(im.sigma + c);
+    // of norm zero) leaves x' = y, whatever g holds: the projection of a start
+    // needs no zeroed g plane.
     const bool stepped = sg != 0.f;  // warp-uniform
-    if (stepped) stage(sg_, gb);
     cp_async_wait_all();
     __syncwarp();
 
@@ -1125,7 +1154,12 @@ __global__ void __launch_bounds__(PW * 32) k_project(const ImgDev *__restrict__ 
     }
     // g is consumed: stage x_k into its plane while the transforms run.
     __syncwarp();
-    stage(sx_, xw);
+    stage([&](int so, long long go) {
+        if constexpr (FIT)
+            cp_async16_l2(sx_ + so, xw + go, policy);
+        else
+            cp_async16(sx_ + so, xw + go);
+    });
     // DCT, columns then rows (dct8x8s); the lane then holds coefficient row j.
     dct8(m);
     transpose8(T0, j, m);
@@ -1173,11 +1207,17 @@ __global__ void __launch_bounds__(PW * 32) k_project(const ImgDev *__restrict__ 
             yn[sx] = fmaf(fnext, xn[sx] - xo[sx], xn[sx]);
         }
         const int o = o0 + k * pitch;
-        if (SH == 1) {
-            xw[o] = xn[0];
+        if constexpr (SH == 1) {
+            if constexpr (FIT)
+                store_l2(xw + o, xn[0], policy);
+            else
+                xw[o] = xn[0];
             yw[o] = yn[0];
         } else {
-            *reinterpret_cast<float2 *>(xw + o) = make_float2(xn[0], xn[SH - 1]);
+            if constexpr (FIT)
+                store_l2(xw + o, make_float2(xn[0], xn[SH - 1]), policy);
+            else
+                *reinterpret_cast<float2 *>(xw + o) = make_float2(xn[0], xn[SH - 1]);
             *reinterpret_cast<float2 *>(yw + o) = make_float2(yn[0], yn[SH - 1]);
         }
     }
@@ -1667,13 +1707,13 @@ struct GraphKey {
     int mode_off[5] = {0, 0, 0, 0, 0};
     uint32_t iterations = 0, tail = 0;
     float tail_stepmul = 1.0f, decay = 0.0f;
-    bool timing = false;
+    bool timing = false, l2_fit = false;
     const void *desc = nullptr, *work = nullptr, *tasks = nullptr;
     bool operator==(const GraphKey &o) const
     {
         return nimg == o.nimg && proj_warps == o.proj_warps && iterations == o.iterations && tail == o.tail &&
                tail_stepmul == o.tail_stepmul && decay == o.decay &&
-               timing == o.timing && desc == o.desc &&
+               timing == o.timing && l2_fit == o.l2_fit && desc == o.desc &&
                work == o.work && tasks == o.tasks && std::equal(wcount, wcount + 12, o.wcount) &&
                std::equal(mode_off, mode_off + 5, o.mode_off);
     }
@@ -1738,6 +1778,7 @@ struct ArtContext {
     int strip_rows_override = 0;      // 0 = tuning cache, else size heuristic
     int sweep_kind_override = 0;
     int proj_warps = art::PROJ_WARPS; // projection warps per block of the current solve
+    bool l2_fit = false;              // its planes nearly fit L2 (l2_fits)
     int proj_warps_override = 0;      // set while the autotuner times a candidate
     std::map<std::string, art::TuneChoice> tune;  // autotuned launch shapes by geometry bucket
     ArtTuneResult last_tune{};        // the last autotune run's choice and timings
@@ -1832,7 +1873,7 @@ constexpr int sweep_smem()
     return SWEEP_WARPS_N * SWEEP_STAGES_N * NCH * SWEEP_CHUNK * (2 * SWEEP_OUT_N + 8) * (int)sizeof(float);
 }
 
-template <int SH, int SV, int PW = PROJ_WARPS>
+template <int SH, int SV, int PW>
 constexpr int proj_smem()
 {
     return PW * 2 * ProjShape<SH, SV>::REGION * (int)sizeof(float);
@@ -1842,17 +1883,14 @@ constexpr int proj_smem()
 // warp takes 4 coefficient blocks of one block row).
 constexpr int PROJ_WARP_CHOICES[3] = {2, 4, 8};
 
-template <int PW>
+template <int PW, bool FIT>
 static cudaError_t set_proj_smem()
 {
-    cudaError_t e = cudaFuncSetAttribute(k_project<1, 1, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         proj_smem<1, 1, PW>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_project<2, 2, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize, proj_smem<2, 2, PW>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_project<2, 1, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize, proj_smem<2, 1, PW>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_project<1, 2, PW>, cudaFuncAttributeMaxDynamicSharedMemorySize, proj_smem<1, 2, PW>());
+    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_project<1, 1, PW, FIT>, a, proj_smem<1, 1, PW>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_project<2, 2, PW, FIT>, a, proj_smem<2, 2, PW>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_project<2, 1, PW, FIT>, a, proj_smem<2, 1, PW>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_project<1, 2, PW, FIT>, a, proj_smem<1, 2, PW>());
     return e;
 }
 
@@ -1887,31 +1925,40 @@ static void launch(Dep dep, void (*k)(P...), int grid, int threads, size_t smem,
     cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
+// Whether the planes of a solve (x, y, g and P, in bytes) are taken to nearly fit
+// L2 (126 MB on two dies). Then what is not read again soon goes first: g once it
+// is read, P once the sweep has read it, x (read and written only by the
+// projection). One iteration without and with: 1920x1080 4:4:4 (100 MB) 55.9 and
+// 52.2 us, 4:2:0 (83 MB) 48.9 and 45.4, 2600x1500 4:4:4 (188 MB) 106.9 and 105.8;
+// 3200x2000 4:2:0 (257 MB) 156.7 and 156.8, 6000x4000 4:4:4 617 and 625. Above
+// the line the projection also reads y and g together and its coefficients last:
+// 6000x4000 4:4:4 617 and 607 us.
+static bool l2_fits(size_t bytes) { return bytes <= ((size_t)200 << 20); }
+
 // One projection launch over n tasks of sampling mode m with PW warps per block.
-template <int PW>
-static void launch_project_mode(Dep dep, int m, int n, const ImgDev *ddesc, const int4 *tk, float fnext,
-                                cudaStream_t s)
+template <int PW, bool FIT>
+static void launch_project_mode(Dep dep, int m, int n, const ImgDev *ddesc, const int4 *tk, float fnext, cudaStream_t s)
 {
     const int grid = (n + PW - 1) / PW;
     if (m == 0)
-        launch(dep, k_project<1, 1, PW>, grid, PW * 32, proj_smem<1, 1, PW>(), s, ddesc, tk, n, fnext);
+        launch(dep, k_project<1, 1, PW, FIT>, grid, PW * 32, proj_smem<1, 1, PW>(), s, ddesc, tk, n, fnext);
     else if (m == 1)
-        launch(dep, k_project<2, 2, PW>, grid, PW * 32, proj_smem<2, 2, PW>(), s, ddesc, tk, n, fnext);
+        launch(dep, k_project<2, 2, PW, FIT>, grid, PW * 32, proj_smem<2, 2, PW>(), s, ddesc, tk, n, fnext);
     else if (m == 2)
-        launch(dep, k_project<2, 1, PW>, grid, PW * 32, proj_smem<2, 1, PW>(), s, ddesc, tk, n, fnext);
+        launch(dep, k_project<2, 1, PW, FIT>, grid, PW * 32, proj_smem<2, 1, PW>(), s, ddesc, tk, n, fnext);
     else
-        launch(dep, k_project<1, 2, PW>, grid, PW * 32, proj_smem<1, 2, PW>(), s, ddesc, tk, n, fnext);
+        launch(dep, k_project<1, 2, PW, FIT>, grid, PW * 32, proj_smem<1, 2, PW>(), s, ddesc, tk, n, fnext);
 }
 
-static void launch_project(Dep dep, int pw, int m, int n, const ImgDev *ddesc, const int4 *tk, float fnext,
-                           cudaStream_t s)
+template <bool FIT>
+static void launch_project(Dep dep, int pw, int m, int n, const ImgDev *ddesc, const int4 *tk, float fnext, cudaStream_t s)
 {
     if (pw == 2)
-        launch_project_mode<2>(dep, m, n, ddesc, tk, fnext, s);
+        launch_project_mode<2, FIT>(dep, m, n, ddesc, tk, fnext, s);
     else if (pw == 8)
-        launch_project_mode<8>(dep, m, n, ddesc, tk, fnext, s);
+        launch_project_mode<8, FIT>(dep, m, n, ddesc, tk, fnext, s);
     else
-        launch_project_mode<4>(dep, m, n, ddesc, tk, fnext, s);
+        launch_project_mode<4, FIT>(dep, m, n, ddesc, tk, fnext, s);
 }
 
 template <int NCH>
@@ -1941,9 +1988,12 @@ int configure_kernels(int device)
     std::lock_guard<std::mutex> lock(mu);
     if ((int)done.size() <= device) done.resize(device + 1, 0);
     if (done[device]) return ART_OK;
-    cudaError_t e = set_proj_smem<2>();
-    if (e == cudaSuccess) e = set_proj_smem<4>();
-    if (e == cudaSuccess) e = set_proj_smem<8>();
+    cudaError_t e = set_proj_smem<2, true>();
+    if (e == cudaSuccess) e = set_proj_smem<4, true>();
+    if (e == cudaSuccess) e = set_proj_smem<8, true>();
+    if (e == cudaSuccess) e = set_proj_smem<2, false>();
+    if (e == cudaSuccess) e = set_proj_smem<4, false>();
+    if (e == cudaSuccess) e = set_proj_smem<8, false>();
     if (e == cudaSuccess) e = set_sweep_smem<1>();
     if (e == cudaSuccess) e = set_sweep_smem<2>();
     if (e == cudaSuccess) e = set_sweep_smem<3>();
@@ -2054,7 +2104,8 @@ static void launch_projections(ArtContext *ctx, float fnext, bool dep = false)
         Dep d;
         d.pdl = dep && !on_side;
         if (dep && on_side && m == last) d.released = ctx->join;
-        launch_project(d, ctx->proj_warps, m, n, ddesc, tasks + ctx->mode_off[m], fnext, on_side ? ctx->side : ctx->stream);
+        const auto go = ctx->l2_fit ? launch_project<true> : launch_project<false>;
+        go(d, ctx->proj_warps, m, n, ddesc, tasks + ctx->mode_off[m], fnext, on_side ? ctx->side : ctx->stream);
     }
     if (split) {
         if (!dep) cudaEventRecord(ctx->join, ctx->side);
@@ -2187,6 +2238,8 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
             }
         }
     }
+    ctx->l2_fit = l2_fits((x_floats + p_floats) * sizeof(float));
+    for (ImgDev &d : ctx->h_desc) d.l2_fit = ctx->l2_fit;
     plan_resident(ctx);
     if ((rc = ctx->xbuf.ensure(x_floats * sizeof(float)))) return rc;
     if ((rc = ctx->coefimg.ensure(coef_bytes))) return rc;
@@ -2368,7 +2421,8 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
             (unsigned long long)(uintptr_t)ctx->net, gen(ctx->net, 0), gen(ctx->net, 1),
             (unsigned long long)(uintptr_t)ctx->net_joint, gen(ctx->net_joint, 0), gen(ctx->net_joint, 1),
             (uintptr_t)ctx->desc.p, (uintptr_t)ctx->tasks.p, (uintptr_t)pred, (uintptr_t)ctx->xbuf.p,
-            (uintptr_t)ctx->coefimg.p, (unsigned long long)nimg, (unsigned long long)ctx->proj_warps};
+            (uintptr_t)ctx->coefimg.p, (unsigned long long)nimg, (unsigned long long)ctx->proj_warps,
+            (unsigned long long)ctx->l2_fit};
         for (int m = 0; m < 5; m++) key.push_back((unsigned long long)ctx->mode_off[m]);
         for (int i = 0; i < nimg; i++) {
             const ImgDev &d = ctx->h_desc[i];
@@ -2627,6 +2681,7 @@ static int run_iterations(ArtContext *ctx, uint32_t iterations, uint32_t tail = 
     key.tail_stepmul = tail_stepmul;
     key.decay = decay;
     key.timing = ctx->timing;
+    key.l2_fit = ctx->l2_fit;
     key.desc = ctx->desc.p;
     key.work = ctx->work.p;
     key.tasks = ctx->tasks.p;
@@ -3817,6 +3872,9 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
             d.invq2[c][j] = 1.0f / (q * q);
         }
     }
+    size_t plane_floats = (size_t)3 * nch * cstride;
+    for (uint32_t c = 0; c < nch; c++) plane_floats += (size_t)ppitch[c] * coefs[c].rounded_px_h;
+    d.l2_fit = l2_fits(plane_floats * sizeof(float));
     ImgDev *ddesc = reinterpret_cast<ImgDev *>(base + o_desc);
     int2 *work = reinterpret_cast<int2 *>(base + o_work);
     int4 *tasks = reinterpret_cast<int4 *>(base + o_tasks);
@@ -3848,16 +3906,8 @@ extern "C" int32_t art_solve_noalloc(uint32_t nchannel, const ArtChannel *coefs,
         for (int m = 3; m >= 0; m--) {
             const int n = mode_off[m + 1] - mode_off[m];
             if (n == 0) continue;
-            const int4 *tk = tasks + mode_off[m];
-            const int grid = (n + PROJ_WARPS - 1) / PROJ_WARPS;
-            if (m == 0)
-                k_project<1, 1><<<grid, PROJ_WARPS * 32, proj_smem<1, 1>(), s>>>(ddesc, tk, n, fnext);
-            else if (m == 1)
-                k_project<2, 2><<<grid, PROJ_WARPS * 32, proj_smem<2, 2>(), s>>>(ddesc, tk, n, fnext);
-            else if (m == 2)
-                k_project<2, 1><<<grid, PROJ_WARPS * 32, proj_smem<2, 1>(), s>>>(ddesc, tk, n, fnext);
-            else
-                k_project<1, 2><<<grid, PROJ_WARPS * 32, proj_smem<1, 2>(), s>>>(ddesc, tk, n, fnext);
+            const auto go = d.l2_fit ? launch_project<true> : launch_project<false>;
+            go(Dep{}, PROJ_WARPS, m, n, ddesc, tasks + mode_off[m], fnext, s);
         }
     }
     NOALLOC_CUDA(cudaGetLastError());

@@ -52,6 +52,7 @@ struct ImgDev {
     float *y;              // FISTA point y_k = x_k + f_k (x_k - x_{k-1})
     float *g;              // gradient planes
     float alpha_tv, alpha_tgv, step;
+    int l2_fit;            // the planes of the solve nearly fit L2 (l2_fits)
     float neg_zero;        // -0.0f, where a kernel needs one that the compiler does not know (f2mul_only)
     float *sigma;          // [4] per channel step / ||g||
     float *partial;        // [ncta * 4] per-block sums of g^2
@@ -158,15 +159,18 @@ __device__ __forceinline__ void dct8(float *a)
 }
 
 // The 8 quantised coefficients of one block row (int16) as floats.
-__device__ __forceinline__ void load_coef_row(const int16_t *row, float *c)
+__device__ __forceinline__ void convert_coef_row(const uint4 &raw, float *c)
 {
-    const uint4 raw = *reinterpret_cast<const uint4 *>(row);
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         c[2 * i] = (float)(int16_t)(w[i] & 0xffffu);
         c[2 * i + 1] = (float)(int16_t)(w[i] >> 16);
     }
+}
+__device__ __forceinline__ void load_coef_row(const int16_t *row, float *c)
+{
+    convert_coef_row(*reinterpret_cast<const uint4 *>(row), c);
 }
 
 // 2-D transforms of a register-resident 8x8 block, columns first then rows,
@@ -264,6 +268,34 @@ __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// L2 policy of data that is not read again soon: marked to be evicted first, or
+// left as it is (then an access with the policy is an ordinary one).
+__device__ __forceinline__ unsigned long long l2_policy(bool first)
+{
+    unsigned long long p, n;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(n));
+    return first ? p : n;
+}
+__device__ __forceinline__ void cp_async16_l2(unsigned smem, const void *gmem, unsigned long long policy)
+{
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "l"(policy)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async16_l2(void *smem, const void *gmem, unsigned long long policy)
+{
+    cp_async16_l2((unsigned)__cvta_generic_to_shared(smem), gmem, policy);
+}
+__device__ __forceinline__ void store_l2(float *p, float v, unsigned long long policy)
+{
+    asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void store_l2(float *p, float2 v, unsigned long long policy)
+{
+    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" ::"l"(p), "f"(v.x), "f"(v.y), "l"(policy)
+                 : "memory");
 }
 
 // Programmatic dependent launch: a kernel launched as a dependent may start

@@ -34,3 +34,19 @@ def test_dependent_launches_equal_ordinary_ones(gpu, name):
         want = ctx.compute_batch(jobs, 12)
     for g in got:
         assert all(np.array_equal(a, b) for pa, pb in zip(g, want) for a, b in zip(pa, pb))
+
+
+def test_planes_beyond_l2_equal_planes_within(gpu, monkeypatch):
+    """The projection stages in another order, and without L2 hints, where the
+    planes of a solve exceed 200 MiB: a batch above the line against its images
+    alone, with the same norm strips."""
+    monkeypatch.setenv("ART_STRIP_ROWS", "32")
+    monkeypatch.setenv("ART_RESIDENT", "0")
+    subs = ["4:2:0", "4:2:2", "4:4:4", "gray"]
+    jobs = [dict(coefs=_jpeg(*SIZES[i % 2], sub, seed=40 + i).coefs) for i, sub in enumerate(subs)]
+    jobs += [dict(coefs=_jpeg(1920, 1080, "4:4:4", seed=50).coefs)] * 3
+    with Context(0) as ctx:
+        got = ctx.compute_batch(jobs, 6)
+        for job, g in zip(jobs[:5], got):
+            alone = ctx.compute_batch([job], 6)[0]
+            assert all(np.array_equal(a, b) for a, b in zip(g, alone))
