@@ -44,11 +44,9 @@ namespace cnn {
 using bf16 = __nv_bfloat16;
 
 constexpr int TPX = 128;                    // output pixels per tile row (MMA M)
-constexpr int TROWS = 2;                    // weight gradient: output rows per tile (the convolution takes 2 or 4)
 constexpr int HPX = TPX + 2;                // halo tile width
-constexpr int HROWS = TROWS + 2;            // weight gradient: halo tile height
-constexpr uint32_t KCOL = HROWS * HPX * 16; // weight gradient: bytes of one 8-channel halo column (8320, 65 x 128)
-constexpr uint32_t DYREG = TROWS * TPX * 16;// bytes of one 8-channel region of a gradient tile (4096)
+constexpr int WTILE = 256;                  // weight gradient: output pixels per tile (rows x columns, wgrad_tile)
+constexpr uint32_t DYREG = WTILE * 16;      // bytes of one 8-channel region of a gradient tile (4096)
 constexpr int THREADS = 192;                // weight gradient: warp 0 loads, warp 1 MMA, warps 2-5 epilogue
 constexpr int CONV_THREADS = 320;           // convolution: warp 0 loads, warp 1 MMA, warps 2-9 epilogue
 constexpr int EPI_THREADS = CONV_THREADS - 64;
@@ -81,6 +79,7 @@ struct ConvArgs {
 struct WgradArgs {
     int B, H, W;
     int cout, cin, nci;  // gradient channels (<= 128), input channels, input channels per CTA (16 or 32)
+    int tpx, trows;      // tile: columns and rows
     int tiles_per_band;
     float *partial;      // [bands][cin/nci][9][cout][nci]
     int stages;
@@ -88,13 +87,14 @@ struct WgradArgs {
     int *err;
 };
 
-__device__ __forceinline__ void tile_coords(int tile, int tiles_x, int tiles_y, int trows, int &b, int &y0, int &x0)
+__device__ __forceinline__ void tile_coords(int tile, int tiles_x, int tiles_y, int trows, int &b, int &y0, int &x0,
+                                            int tpx = TPX)
 {
     const int per = tiles_x * tiles_y;
     b = tile / per;
     const int r = tile - b * per;
     y0 = (r / tiles_x) * trows;
-    x0 = (r % tiles_x) * TPX;
+    x0 = (r % tiles_x) * tpx;
 }
 
 // Waits without honouring the abort flag (used to drain in-flight work
@@ -416,6 +416,18 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) k_conv3x3(const __grid_consta
     if (threadIdx.x == 0 && abort_s) atomicExch(a.err, 1);
 }
 
+// Weight gradient partials of a band of tiles for one chunk of nci input channels.
+//
+// An accumulator is dY^T X of one tap: M = the gradient channels (padded to 128),
+// N = nci, K = a tile's pixels. An MMA of N = 32 takes as long as one of N = 96:
+// its A operand (128 x 16) has to come through shared memory either way. So the
+// three taps of a tap column are one MMA of N = 3 nci. The halo tile is laid out
+// [row][8-channel group][column] by one 5-D copy; the operand's 8-channel groups
+// of tap rows 0, 1 and 2 are then equally spaced (columns x 16 bytes), and
+// tap column tx starts tx pixels further on. Accumulator columns: [tx][ty][c].
+//
+// Tiles are 256 pixels of 128, 64 or 32 columns (wgrad_tile): a tile wider than the
+// tensor is work for nothing. One wave of blocks (each holds all of TMEM).
 __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__ CUtensorMap dymap,
                                                          const __grid_constant__ CUtensorMap xmap, const WgradArgs a)
 {
@@ -427,12 +439,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
     volatile int *abort_p = &abort_s;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_x = (a.W + TPX - 1) / TPX, tiles_y = (a.H + TROWS - 1) / TROWS;
+    const int tpx = a.tpx, hpx = tpx + 2, G = a.nci / 8;
+    const int tiles_x = (a.W + tpx - 1) / tpx, tiles_y = (a.H + a.trows - 1) / a.trows;
     const int ntiles = a.B * tiles_x * tiles_y;
     const int band = blockIdx.x, chunk = blockIdx.y, nchunk = gridDim.y;
     const int t_begin = band * a.tiles_per_band, t_end = min(ntiles, t_begin + a.tiles_per_band);
     const int S = a.stages;
-    const uint32_t dy_bytes = 16 * DYREG;  // M = 128 gradient channels: 16 regions (unused ones are never read back)
+    // M = 128 gradient channels are read as 16 regions. Those past cout / 8 are
+    // whatever follows in shared memory (the host leaves room for them); their
+    // rows of the accumulators are never read back.
+    const uint32_t dy_bytes = (uint32_t)(a.cout / 8) * DYREG;
 
     if (threadIdx.x == 0) {
         abort_s = 0;
@@ -452,21 +468,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t tx_bytes = (uint32_t)(a.cout / 8) * DYREG + (uint32_t)(a.nci / 8) * KCOL;
+            const uint32_t tx_bytes = dy_bytes + (uint32_t)((a.trows + 2) * G * hpx * 16);
             uint32_t it = 0;
             for (int tile = t_begin; tile < t_end; tile++, it++) {
                 const int s = it % S;
                 const uint32_t use = it / S;
                 if (use > 0 && !tc::mbar_wait(&empty_bar[s], (use - 1) & 1, abort_p)) break;
                 int b, y0, x0;
-                tile_coords(tile, tiles_x, tiles_y, TROWS, b, y0, x0);
+                tile_coords(tile, tiles_x, tiles_y, a.trows, b, y0, x0, tpx);
                 unsigned char *st = smem + (size_t)s * a.stage_bytes;
                 tc::mbar_arrive_expect_tx(&full_bar[s], tx_bytes);
                 for (int g = 0; g < a.cout / 8; g++)
                     tc::tma_load_4d(st + g * DYREG, &dymap, 8 * g, x0, y0, b, &full_bar[s]);
-                for (int j = 0; j < a.nci / 8; j++)
-                    tc::tma_load_4d(st + dy_bytes + j * KCOL, &xmap, chunk * a.nci + 8 * j, x0 - 1, y0 - 1, b,
-                                    &full_bar[s]);
+                tc::tma_load_5d(st + dy_bytes, &xmap, 0, x0 - 1, chunk * G, y0 - 1, b, &full_bar[s]);
             }
             const uint32_t last = it;
             for (uint32_t k = (last > (uint32_t)S ? last - S : 0); k < last; k++)
@@ -475,7 +489,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
         __syncwarp();
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = tc::idesc_bf16(128, a.nci, 1, 1);
+            const uint32_t idesc = tc::idesc_bf16(128, 3 * a.nci, 1, 1);
+            const int sh = 31 - __clz(tpx);  // log2
             uint32_t it = 0;
             bool ok = true;
             for (int tile = t_begin; tile < t_end; tile++, it++) {
@@ -487,19 +502,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
                 tc::tc_fence_after();
                 const uint32_t st = tc::smem_u32(smem + (size_t)s * a.stage_bytes);
                 const uint32_t xs = st + dy_bytes;
-                for (int tap = 0; tap < 9; tap++) {
-                    const int ty = tap / 3, tx = tap % 3;
-#pragma unroll
-                    for (int r = 0; r < TROWS; r++)
-#pragma unroll
-                        for (int k0 = 0; k0 < TPX; k0 += 16) {
-                            const uint64_t adesc = tc::smem_desc(st + (uint32_t)((r * TPX + k0) * 16), 128, DYREG);
-                            const uint64_t bdesc =
-                                tc::smem_desc(xs + (uint32_t)(((r + ty) * HPX + k0 + tx) * 16), 128, KCOL);
-                            tc::mma_bf16(tbase + (uint32_t)(tap * a.nci), adesc, bdesc, idesc,
-                                         (it | r | k0) != 0);
-                        }
-                }
+                for (int tx = 0; tx < 3; tx++)
+#pragma unroll 4
+                    for (int p = 0; p < WTILE; p += 16) {
+                        const int r = p >> sh, k0 = p & (tpx - 1);
+                        const uint64_t adesc = tc::smem_desc(st + (uint32_t)(p * 16), 128, DYREG);
+                        const uint64_t bdesc =
+                            tc::smem_desc(xs + (uint32_t)((r * G * hpx + k0 + tx) * 16), 128, (uint32_t)(hpx * 16));
+                        tc::mma_bf16(tbase + (uint32_t)(tx * 3 * a.nci), adesc, bdesc, idesc, (it | p) != 0);
+                    }
                 tc::mma_commit(&empty_bar[s]);
             }
             if (ok) tc::mma_commit(&accf_bar);
@@ -521,7 +532,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
 #pragma unroll 1
                 for (int c0 = 0; c0 < a.nci; c0 += 16) {
                     float v[16];
-                    tc::tmem_ld16(tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)(tap * a.nci + c0), v);
+                    tc::tmem_ld16(tbase + ((uint32_t)(q * 32) << 16) +
+                                      (uint32_t)((tap % 3 * 3 + tap / 3) * a.nci + c0), v);
                     if (co < a.cout) {
                         float4 *o = reinterpret_cast<float4 *>(dst + ((size_t)tap * a.cout + co) * a.nci + c0);
 #pragma unroll
@@ -541,19 +553,29 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
     if (threadIdx.x == 0 && abort_s) atomicExch(a.err, 1);
 }
 
-// dW[n][tap][c] (+)= sum over bands of the partials, in band order.
-__global__ void k_wgrad_reduce(const float *__restrict__ partial, int bands, int cout, int cin, int nci,
-                               float *__restrict__ dw, int accumulate)
+// dW[n][tap][c] (+)= sum over bands of the partials. Bound by latency (a few MB
+// in all): a block takes 32 neighbouring partials, each of its eight warps an
+// eighth of the bands, and adds the warps' sums in order. One thread an output
+// took 11 to 27 us with up to 256 bands.
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ partial, int bands, int cout, int cin,
+                                                      int nci, float *__restrict__ dw, int accumulate)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int total = cout * 9 * cin;
-    if (i >= total) return;
-    const int c = i % cin, tap = (i / cin) % 9, n = i / (9 * cin);
-    const int chunk = c / nci, cc = c % nci, nchunk = cin / nci;
-    float s = 0.f;
-    for (int b = 0; b < bands; b++)
-        s += partial[(((size_t)(b * nchunk + chunk) * 9 + tap) * cout + n) * nci + cc];
-    dw[i] = accumulate ? dw[i] + s : s;
+    __shared__ float s[8][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int total = cout * 9 * cin;  // a multiple of 32
+    const int e = blockIdx.x * 32 + lane;  // index of a band's partials [chunk][tap][n][cc]
+    float t = 0.f;
+#pragma unroll 8
+    for (int b = warp; b < bands; b += 8) t += partial[(size_t)b * total + e];
+    s[warp][lane] = t;
+    __syncthreads();
+    if (warp) return;
+    t = s[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; w++) t += s[w][lane];
+    const int cc = e % nci, n = e / nci % cout, tap = e / (nci * cout) % 9, chunk = e / (nci * cout * 9);
+    float *o = dw + ((size_t)n * 9 + tap) * cin + chunk * nci + cc;
+    *o = accumulate ? *o + t : t;
 }
 
 // Packs fp32 master weights W[cout][9][cin] into the bf16 layout a conv stage
@@ -704,33 +726,58 @@ __global__ void k_unpool_add_mask(bf16 *__restrict__ g, const bf16 *__restrict__
 }
 
 // Per-channel sums over all pixels of g[npix][C] (bias gradient), two passes
-// with a fixed order: blocks write partials, one block adds them.
-__global__ void k_colsum_partial(const bf16 *__restrict__ g, long long npix, int C, float *__restrict__ partial)
+// with a fixed order: blocks write partials, one block adds them. Both are
+// bound by latency unless many loads are in flight: the first pass reads
+// 16-byte pieces of eight channels where C and g allow it (single channels took
+// 11 us for 16 MB), the second one takes every thread of its block for the partials
+// (a thread a channel took 13 us).
+__device__ __forceinline__ void colsum_rows(const float *s, int rows, int C, float *out, int accumulate)
 {
-    __shared__ float s[256];
-    const int per_row = 256 / C;  // pixels handled per step by the block
-    const int c = threadIdx.x % C, r = threadIdx.x / C;
-    float acc = 0.f;
-    if (r < per_row)
-        for (long long p = (long long)blockIdx.x * per_row + r; p < npix; p += (long long)gridDim.x * per_row)
-            acc += __bfloat162float(g[p * C + c]);
-    s[threadIdx.x] = acc;
+    __shared__ float part[1024];
+    const int c = threadIdx.x % C, k = threadIdx.x / C, P = blockDim.x / C;
+    float t = 0.f;
+    if (k < P)
+        for (int r = k; r < rows; r += P) t += s[r * C + c];
+    part[threadIdx.x] = t;
     __syncthreads();
-    if (threadIdx.x < C) {
-        float t = 0.f;
-        for (int k = 0; k < per_row; k++) t += s[k * C + threadIdx.x];
-        partial[(size_t)blockIdx.x * C + threadIdx.x] = t;
-    }
+    if (threadIdx.x >= C) return;
+    for (int q = 1; q < P; q++) t += part[q * C + c];
+    out[c] = accumulate ? out[c] + t : t;
 }
 
-__global__ void k_colsum_final(const float *__restrict__ partial, int nblk, int C, float *__restrict__ out,
-                               int accumulate)
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_colsum_partial(const bf16 *__restrict__ g, long long npix, int C,
+                                                        float *__restrict__ partial)
 {
-    const int c = threadIdx.x;
-    if (c >= C) return;
-    float t = 0.f;
-    for (int b = 0; b < nblk; b++) t += partial[(size_t)b * C + c];
-    out[c] = accumulate ? out[c] + t : t;
+    constexpr int E = VEC ? 8 : 1;
+    __shared__ float s[256 * E];
+    const int groups = C / E, rows = 256 / groups;  // rows: pixels handled per step by the block
+    const int c = threadIdx.x % groups, r = threadIdx.x / groups;
+    float acc[E] = {};
+    if (r < rows) {
+        const long long step = (long long)gridDim.x * rows;
+#pragma unroll 4
+        for (long long p = (long long)blockIdx.x * rows + r; p < npix; p += step) {
+            if constexpr (VEC) {
+                const uint4 v4 = __ldg(reinterpret_cast<const uint4 *>(g + p * C) + c);
+                const bf16 *v = reinterpret_cast<const bf16 *>(&v4);
+#pragma unroll
+                for (int i = 0; i < E; i++) acc[i] += __bfloat162float(v[i]);
+            } else {
+                acc[0] += __bfloat162float(g[p * C + c]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < E; i++) s[r * C + c * E + i] = acc[i];
+    }
+    __syncthreads();
+    colsum_rows(s, rows, C, partial + (size_t)blockIdx.x * C, 0);
+}
+
+__global__ void __launch_bounds__(1024) k_colsum_final(const float *__restrict__ partial, int nblk, int C,
+                                                       float *__restrict__ out, int accumulate)
+{
+    colsum_rows(partial, nblk, C, out, accumulate);
 }
 
 // Network input from a coefficient image: per 8x8 block the decoded samples
@@ -1253,7 +1300,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 // NHWC bf16 tensor map with boxes of bc channels x bw pixels x bh rows; bc = 8
 // unswizzled, 16 with the 32-byte swizzle, 32 with the 64-byte swizzle.
 bool make_map(CUtensorMap *m, const void *base, int B, int H, int W, int C, int bw, int bh, std::string &err,
-              int bc = 8)
+              int bc = 8, int groups = 0)
 {
     auto fn = encode_fn();
     if (!fn) {
@@ -1264,14 +1311,21 @@ bool make_map(CUtensorMap *m, const void *base, int B, int H, int W, int C, int 
         err = "tensor base must be 16-byte aligned and channels a multiple of 8";
         return false;
     }
-    cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    cuuint32_t box[4] = {(cuuint32_t)bc, (cuuint32_t)bw, (cuuint32_t)bh, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
+    const cuuint64_t c = C, w = W, h = H, n = B;
+    cuuint64_t dims[5] = {c, w, h, n, 1}, strides[4] = {c * 2, w * c * 2, h * w * c * 2, 0};
+    cuuint32_t box[5] = {(cuuint32_t)bc, (cuuint32_t)bw, (cuuint32_t)bh, 1, 1};
+    cuuint32_t es[5] = {1, 1, 1, 1, 1};
+    if (groups) {  // 8-channel groups as a dimension of their own: {8, W, C / 8, H, B}
+        const cuuint64_t gd[5] = {8, w, c / 8, h, n}, gs[4] = {c * 2, 16, w * c * 2, h * w * c * 2};
+        const cuuint32_t gb[5] = {8, (cuuint32_t)bw, (cuuint32_t)groups, (cuuint32_t)bh, 1};
+        std::copy(gd, gd + 5, dims);
+        std::copy(gs, gs + 4, strides);
+        std::copy(gb, gb + 5, box);
+    }
     const CUtensorMapSwizzle sw = bc == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
                                   : bc == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
                                              : CU_TENSOR_MAP_SWIZZLE_NONE;
-    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, box, es,
+    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, groups ? 5 : 4, const_cast<void *>(base), dims, strides, box, es,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -1418,6 +1472,22 @@ int32_t conv3x3(const ArtCnnConv *d, cudaStream_t s)
     return check_launch("k_conv3x3");
 }
 
+// Tiles of the weight gradient, and their width: of 128, 64 and 32 columns the
+// one with the fewest tiles (the widest of equals, its halo is the smallest).
+// Tensors of 64 and 32 columns (the lower levels of 256-pixel crops) took two and
+// four times as many tiles of 128 columns.
+long long wgrad_tiles(int B, int H, int W, int tpx)
+{
+    return (long long)B * ((H + WTILE / tpx - 1) / (WTILE / tpx)) * ((W + tpx - 1) / tpx);
+}
+int wgrad_tile(int B, int H, int W)
+{
+    int best = 128;
+    for (int t : {64, 32})
+        if (wgrad_tiles(B, H, W, t) < wgrad_tiles(B, H, W, best)) best = t;
+    return best;
+}
+
 int32_t wgrad3x3(const ArtCnnWgrad *d, cudaStream_t s)
 {
     if (!d || !d->x || !d->dy || !d->dw || !d->workspace || !d->err)
@@ -1426,9 +1496,10 @@ int32_t wgrad3x3(const ArtCnnWgrad *d, cudaStream_t s)
     if (d->cout < 8 || d->cout > 128 || d->cout % 8) return fail(ART_ERR_INVALID_ARGUMENT, "wgrad: cout must be 8..128, multiple of 8");
     const int nci = d->cin % 32 == 0 ? 32 : 16;
     if (d->cin < 16 || d->cin % 16) return fail(ART_ERR_INVALID_ARGUMENT, "wgrad: cin must be a multiple of 16");
-    const long long ntiles = (long long)d->B * ((d->H + TROWS - 1) / TROWS) * ((d->W + TPX - 1) / TPX);
+    const int tpx = wgrad_tile(d->B, d->H, d->W), trows = WTILE / tpx;
+    const long long ntiles = wgrad_tiles(d->B, d->H, d->W, tpx);
     const int nchunk = d->cin / nci;
-    int bands = (int)std::max<long long>(1, std::min<long long>(ntiles, (2LL * num_sms() + nchunk - 1) / nchunk));
+    int bands = (int)std::max<long long>(1, std::min<long long>(ntiles, num_sms() / nchunk));
     const long long per_band_bytes = (long long)nchunk * 9 * d->cout * nci * 4;
     bands = (int)std::min<long long>(bands, std::max<long long>(1, (long long)d->workspace_bytes / per_band_bytes));
     if (per_band_bytes > (long long)d->workspace_bytes) return fail(ART_ERR_INVALID_ARGUMENT, "wgrad: workspace too small");
@@ -1436,8 +1507,9 @@ int32_t wgrad3x3(const ArtCnnWgrad *d, cudaStream_t s)
     bands = (int)((ntiles + tpb - 1) / tpb);
     CUtensorMap dymap, xmap;
     std::string err;
-    if (!make_map(&dymap, d->dy, d->B, d->H, d->W, d->cout, TPX, TROWS, err)) return fail(ART_ERR_CUDA, "wgrad: " + err);
-    if (!make_map(&xmap, d->x, d->B, d->H, d->W, d->cin, HPX, HROWS, err)) return fail(ART_ERR_CUDA, "wgrad: " + err);
+    if (!make_map(&dymap, d->dy, d->B, d->H, d->W, d->cout, tpx, trows, err)) return fail(ART_ERR_CUDA, "wgrad: " + err);
+    if (!make_map(&xmap, d->x, d->B, d->H, d->W, d->cin, tpx + 2, trows + 2, err, 8, nci / 8))
+        return fail(ART_ERR_CUDA, "wgrad: " + err);
     WgradArgs a{};
     a.B = d->B;
     a.H = d->H;
@@ -1447,15 +1519,21 @@ int32_t wgrad3x3(const ArtCnnWgrad *d, cudaStream_t s)
     a.nci = nci;
     a.tiles_per_band = tpb;
     a.partial = static_cast<float *>(d->workspace);
-    a.stage_bytes = 16 * DYREG + (uint32_t)(nci / 8) * KCOL;
-    a.stages = (int)std::min<uint32_t>(MAX_STAGES, SMEM_BUDGET / a.stage_bytes);
+    a.tpx = tpx;
+    a.trows = trows;
+    const uint32_t halo = (uint32_t)((trows + 2) * (nci / 8) * (tpx + 2) * 16);
+    a.stage_bytes = ((uint32_t)(d->cout / 8) * DYREG + halo + 1023u) / 1024u * 1024u;
+    // The last stage's 16 gradient regions end past the stage where cout < 128.
+    const uint32_t tail = std::max(a.stage_bytes, 16 * DYREG);
+    a.stages = (int)std::min<uint32_t>(MAX_STAGES, (SMEM_BUDGET - tail) / a.stage_bytes + 1);
+    const uint32_t smem = (a.stages - 1) * a.stage_bytes + tail + 1024;
     a.err = d->err;
     set_smem_attribute_once(reinterpret_cast<const void *>(k_wgrad3x3), 1);
-    k_wgrad3x3<<<dim3(bands, nchunk), THREADS, a.stages * a.stage_bytes + 1024, s>>>(dymap, xmap, a);
+    k_wgrad3x3<<<dim3(bands, nchunk), THREADS, smem, s>>>(dymap, xmap, a);
     int32_t rc = check_launch("k_wgrad3x3");
     if (rc) return rc;
     const int total = d->cout * 9 * d->cin;
-    k_wgrad_reduce<<<(total + 255) / 256, 256, 0, s>>>(a.partial, bands, d->cout, d->cin, nci, d->dw, d->accumulate);
+    k_wgrad_reduce<<<total / 32, 256, 0, s>>>(a.partial, bands, d->cout, d->cin, nci, d->dw, d->accumulate);
     return check_launch("k_wgrad_reduce");
 }
 
@@ -1542,10 +1620,12 @@ int32_t art_cnn_bias_grad(const void *g, int64_t npix, int32_t C, float *workspa
     int nblk = (int)std::min<long long>(2 * num_sms(), workspace_bytes / (4LL * C));
     if (nblk < 1) return fail(ART_ERR_INVALID_ARGUMENT, "bias_grad: workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    k_colsum_partial<<<nblk, 256, 0, s>>>(static_cast<const bf16 *>(g), npix, C, workspace);
+    const bool vec = C % 8 == 0 && (reinterpret_cast<uintptr_t>(g) & 15) == 0;
+    const auto pass = vec ? k_colsum_partial<true> : k_colsum_partial<false>;
+    pass<<<nblk, 256, 0, s>>>(static_cast<const bf16 *>(g), npix, C, workspace);
     int32_t rc = check_launch("k_colsum_partial");
     if (rc) return rc;
-    k_colsum_final<<<1, 256, 0, s>>>(workspace, nblk, C, out, accumulate);
+    k_colsum_final<<<1, 1024, 0, s>>>(workspace, nblk, C, out, accumulate);
     return check_launch("k_colsum_final");
 }
 
