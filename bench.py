@@ -1191,7 +1191,7 @@ def main():
 
     modes = len({(c.horizontal_samp_factor, c.vertical_samp_factor) for j in jpegs for c in j.coefs})
     nchs = len({j.nchannel for j in jpegs})
-    per_step = sum(j.nchannel for j in jpegs) + 1 + (nchs + modes) * iters
+    per_step = 1 + (nchs + modes) * iters
     if rank == 0:
         line = {
             "metric": wl["metric"], "value": value, "unit": "MPix/s", "n_gpus": world, "steps": args.steps,
