@@ -31,6 +31,7 @@
 
 #include "../../include/artefact_b200.h"
 #include "art_internal.h"
+#include "growbuf.h"
 #include "solver_kernels.cuh"
 
 namespace art {
@@ -1588,69 +1589,29 @@ int fail(int code, const std::string &msg)
             return fail(ART_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));   \
     } while (0)
 
-// A device buffer that only grows. It grows by at least half its size (in
-// 2 MiB steps), so a stream of solves of slowly growing size -- batches of a
-// decode pipeline -- reallocates rarely: cudaFree waits for the whole device,
-// which would serialise contexts working side by side, and a new address
-// forces the iteration graph to be captured again.
-struct DevBuf {
-    void *p = nullptr;
-    size_t n = 0;
-    int ensure(size_t bytes)
+// Device memory of the solver, and pinned host memory: host-device copies from
+// that run asynchronously at full link speed, where pageable ones are staged by
+// the driver one call at a time.
+struct DeviceMem {
+    static int alloc(void **p, size_t bytes)
     {
-        if (bytes <= n) return ART_OK;
-        if (n) bytes = std::max(bytes, n + n / 2);
-        bytes = (bytes + (2u << 20) - 1) / (2u << 20) * (2u << 20);
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            return fail(ART_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        }
-        n = bytes;
-        return ART_OK;
+        const cudaError_t e = cudaMalloc(p, bytes);
+        return e == cudaSuccess ? ART_OK : fail(ART_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
-    void release()
-    {
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
-    }
+    static void free(void *p) { cudaFree(p); }
 };
+struct PinnedMem {
+    static int alloc(void **p, size_t bytes)
+    {
+        const cudaError_t e = cudaHostAlloc(p, bytes, cudaHostAllocDefault);
+        return e == cudaSuccess ? ART_OK : fail(ART_ERR_CUDA, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
+    }
+    static void free(void *p) { cudaFreeHost(p); }
+};
+using DevBuf = GrowBuf<DeviceMem>;
+using HostBuf = GrowBuf<PinnedMem>;
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
-
-// Pinned host buffer that only grows, like DevBuf: host-device copies from it
-// run asynchronously at full link speed, where pageable ones are staged by the
-// driver one call at a time.
-struct HostBuf {
-    void *p = nullptr;
-    size_t n = 0;
-    int ensure(size_t bytes)
-    {
-        if (bytes <= n) return ART_OK;
-        if (n) bytes = std::max(bytes, n + n / 2);
-        bytes = (bytes + (2u << 20) - 1) / (2u << 20) * (2u << 20);
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        n = 0;
-        cudaError_t e = cudaHostAlloc(&p, bytes, cudaHostAllocDefault);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            return fail(ART_ERR_CUDA, std::string("cudaHostAlloc: ") + cudaGetErrorString(e));
-        }
-        n = bytes;
-        return ART_OK;
-    }
-    void release()
-    {
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        n = 0;
-    }
-};
 
 struct CopyJob {
     void *dst;
@@ -2248,14 +2209,15 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
     if ((rc = ctx->desc.ensure(nimg * sizeof(ImgDev)))) return rc;
     if (ctx->resident && !ctx->res_cluster) {
         // Exchange words of the on-chip solver. Tags only ever grow, so words of
-        // earlier solves never match; new memory and a wrapped count start at zero.
+        // earlier solves never match; new memory, which may hold any word, and a
+        // wrapped count start at zero.
         ImgDev &d = ctx->h_desc[0];
         const size_t part = align_up((size_t)d.nstrips * d.nch * 2 * sizeof(unsigned long long), 256) + 256;
         const size_t need = part + (size_t)d.nch * d.cstride * sizeof(unsigned long long);
-        const void *before = ctx->res_xchg.p;
         if ((rc = ctx->res_xchg.ensure(need))) return rc;
-        if (ctx->res_xchg.p != before || ctx->res_epoch > 0xffffffffu - iterations - 2u) {
+        if (ctx->res_xchg.fresh || ctx->res_epoch > 0xffffffffu - iterations - 2u) {
             ART_CUDA(cudaMemsetAsync(ctx->res_xchg.p, 0, ctx->res_xchg.n, ctx->stream));
+            ctx->res_xchg.fresh = false;
             ctx->res_epoch = 0;
         }
         d.res_part = static_cast<unsigned long long *>(ctx->res_xchg.p);
