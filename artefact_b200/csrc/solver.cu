@@ -2108,12 +2108,17 @@ static int resident_tiles(ImgDev &d, int rows)
 // than 1 us through L2 (96x64 4:2:0: 476 against 552 us), but not at the price of
 // taller tiles (200x136, 18 tiles of 16 rows or 10 of 32: 620 against 800 us).
 // ART_RESIDENT=0 turns the on-chip solver off, 1 keeps it from forming clusters.
+// A call that the caller's own stream capture has reached gets the launch pair,
+// whose graph launch CUDA refuses there: a replayed on-chip launch would find
+// its own tags in the exchange words and wait for nothing.
 static void plan_resident(ArtContext *ctx)
 {
     ctx->resident = ctx->res_cluster = false;
     const char *er = getenv("ART_RESIDENT");
     const int env = er ? atoi(er) : 2;
     if (ctx->h_desc.size() != 1 || ctx->timing || env == 0) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
     ImgDev &d = ctx->h_desc[0];
     if (d.sweep_kind != 0 || d.nstrips > 8 * RES_GROUPS) return;
     const int sms = multiprocessors(ctx->device);

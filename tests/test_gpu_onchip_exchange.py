@@ -3,9 +3,12 @@
 Tagged words decide when a block goes on, so no word may carry a tag that its
 solve still waits for.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
+from artefact_b200 import _native as N
 from artefact_b200 import synth
 from artefact_b200.api import Context, Jpeg, JpegSource
 
@@ -49,3 +52,45 @@ def test_grown_exchange_memory_starts_at_zero(gpu, monkeypatch):
         for j, w in zip(jpegs, want):
             _leave_tagged_words()
             assert _equal(_solve(ctx, j), w), (j.real_px_w, j.real_px_h)
+
+
+@pytest.mark.parametrize("size,sub", [((96, 64), "4:2:0"), ((518, 389), "gray")])
+def test_callers_capture_is_refused(gpu, size, sub):
+    """A solve cannot be captured into the caller's graph, on chip no more than
+    as launch pairs: the graph would carry this call's tags."""
+    import torch
+
+    j = _jpeg(*size, sub)
+    W, H, _ = j.max_rounded()
+    ch, keep = (N.ArtChannel * j.nchannel)(), []
+    for a, co in zip(ch, j.coefs):
+        buf, q = torch.from_numpy(co.dct_coefs.astype(np.int16)).cuda(), np.ascontiguousarray(co.quant_table, np.float32)
+        keep += [buf, q]
+        a.rounded_px_w, a.rounded_px_h, a.block_w, a.block_h = co.rounded_px_w, co.rounded_px_h, co.block_w, co.block_h
+        a.samp_h, a.samp_v = co.horizontal_samp_factor, co.vertical_samp_factor
+        a.coef_type, a.dct_coefs = N.ART_COEF_I16, buf.data_ptr()
+        a.quant_table = q.ctypes.data_as(C.POINTER(C.c_float))
+    outs = [torch.empty(H, W, device="cuda") for _ in range(j.nchannel)]
+    ptrs = (C.c_void_p * j.nchannel)(*[o.data_ptr() for o in outs])
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def call(ctx):
+        return N.lib().art_context_compute_device(ctx.handle, j.nchannel, ch, 0.3, (C.c_float * 3)(*[0.001] * 3), 7,
+                                                  W, H, ptrs, W, None, C.c_void_p(stream.cuda_stream))
+
+    rcs = []
+    with Context(0) as ctx:
+        want = _solve(ctx, j)
+        for _ in range(2):  # with everything allocated, nothing else stands in the way
+            N.check(call(ctx))
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError):  # the refused launch invalidates the capture
+            with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=stream, capture_error_mode="thread_local"):
+                rcs.append(call(ctx))
+    assert rcs == [N.ART_ERR_CUDA]
+    with Context(0) as ctx:
+        call(ctx)  # reports the refused launch once more
+        N.check(call(ctx))
+        torch.cuda.synchronize()
+    assert all(np.array_equal(o.cpu().numpy().ravel(), w) for o, w in zip(outs, want))
