@@ -40,7 +40,7 @@ constexpr int RES_STRIP = 28;          // columns of a norm strip (SWEEP_OUT_N)
 constexpr int RES_CLUSTER_STRIPS = 256;                 // norm strips of an image solved by one cluster, at most
 constexpr int RES_GROUPS = 512;                         // groups of eight norm strips of an image, at most
 constexpr unsigned RES_ERR_TIMEOUT = 2u;                // bit of the solve's error flag
-constexpr long long RES_WAIT_LIMIT = 4000000000LL;      // clock cycles a barrier wait may take (about 2 s)
+constexpr long long RES_WAIT_LIMIT = 4000000000LL;      // clock cycles a wait of a solve may take (about 2 s)
 
 // Shared-memory layout of one tile (offsets in floats; coef in int16 from its
 // own float offset).
@@ -83,7 +83,8 @@ __host__ __device__ inline ResLayout res_layout(const ImgDev &im)
 // two ahead, since it needs everybody's partials in between); border pixels
 // are not: the next ones are sent only after everybody's next partials, which
 // follow their reading. Polls are bounded: a block that gives up raises the
-// error flag and leaves, and so, one after the other, do those that wait for it.
+// error flag and leaves without posting what it could not form, and so do those
+// that wait for it.
 __device__ __forceinline__ void res_cluster_sync()
 {
     __syncwarp();
@@ -104,10 +105,10 @@ __device__ __forceinline__ unsigned long long res_peek(const unsigned long long 
     return v;
 }
 
-// Gives up a wait that has lasted too long.
-__device__ __forceinline__ bool res_gave_up(long long t0, int *s_abort, unsigned *err)
+// Gives up a wait that has lasted longer than `limit` clock cycles.
+__device__ __forceinline__ bool res_gave_up(long long t0, long long limit, int *s_abort, unsigned *err)
 {
-    if (clock64() - t0 <= RES_WAIT_LIMIT) return false;
+    if (clock64() - t0 <= limit) return false;
     *s_abort = 1;
     atomicOr(err, RES_ERR_TIMEOUT);
     return true;
@@ -384,7 +385,7 @@ template <int NCH, bool CLUSTER>
 __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__restrict__ imgs,
                                                              const int2 *__restrict__ work,
                                                              const float2 *__restrict__ sched, int iterations,
-                                                             unsigned epoch, unsigned *err)
+                                                             unsigned epoch, long long wait_limit, unsigned *err)
 {
     extern __shared__ float4 s_dyn[];
     __shared__ double s_dred[8][NCH];
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
                             for (int c = 0; c < NCH; c++) v[c] = res_peek(part + c * n + i);
 #pragma unroll
                             for (int c = 0; c < NCH; c++) all &= (unsigned)(v[c] >> 32) == tag;
-                            if (all || res_gave_up(t0, &s_abort, err)) break;
+                            if (all || res_gave_up(t0, wait_limit, &s_abort, err)) break;
                         }
 #pragma unroll
                         for (int c = 0; c < NCH; c++) e[c] = __uint_as_float((unsigned)v[c]);
@@ -562,13 +563,14 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
             if (tid < NCH) {
                 const float sg = sigma_final<NCH>(s_dred, tid, im.step * sc.y);
                 s_sigma[tid] = sg;
-                if constexpr (!CLUSTER) res_post(im.res_sigma + tid, sg, tag);
+                // Sums of which some never came are nobody's step.
+                if (!CLUSTER && !s_abort) res_post(im.res_sigma + tid, sg, tag);
             }
         } else if (tid < NCH) {
             const long long t0 = clock64();
             unsigned long long v;
             do v = res_peek(im.res_sigma + tid);
-            while ((unsigned)(v >> 32) != tag && !res_gave_up(t0, &s_abort, err));
+            while ((unsigned)(v >> 32) != tag && !res_gave_up(t0, wait_limit, &s_abort, err));
             s_sigma[tid] = __uint_as_float((unsigned)v);
         }
         __syncthreads();
@@ -626,7 +628,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
                     }
 #pragma unroll
                     for (int i = 0; i < 4; i++) all &= (unsigned)(v[i] >> 32) == tag && (unsigned)(w[i] >> 32) == tag;
-                    if (all || res_gave_up(t0, &s_abort, err)) break;
+                    if (all || res_gave_up(t0, wait_limit, &s_abort, err)) break;
                 }
 #pragma unroll
                 for (int i = 0; i < 4; i++) {

@@ -2552,7 +2552,8 @@ static std::vector<float2> iteration_schedule(uint32_t iterations, uint32_t tail
 }
 
 template <int NCH, bool CLUSTER>
-static cudaError_t launch_resident(ArtContext *ctx, int blocks, int cluster, size_t smem, int iterations)
+static cudaError_t launch_resident(ArtContext *ctx, int blocks, int cluster, size_t smem, int iterations,
+                                   long long wait_limit = RES_WAIT_LIMIT)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
@@ -2572,17 +2573,14 @@ static cudaError_t launch_resident(ArtContext *ctx, int blocks, int cluster, siz
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_resident<NCH, CLUSTER>, static_cast<const ImgDev *>(ctx->desc.p),
                               static_cast<const int2 *>(ctx->res_work.p), static_cast<const float2 *>(ctx->res_sched.p),
-                              iterations, ctx->res_epoch, ctx->errflag);
+                              iterations, ctx->res_epoch, wait_limit, ctx->errflag);
 }
 
-// The iteration loop of the current solve as one on-chip launch.
-static int run_resident(ArtContext *ctx, const std::vector<float2> &sched)
+// Uploads the blocks {image, tile} and the schedule of an on-chip launch where
+// they are not what the device holds.
+static int upload_resident(ArtContext *ctx, int blocks, const std::vector<float2> &sched)
 {
     int rc;
-    const ImgDev &d = ctx->h_desc[0];
-    int cluster = 1;
-    while (cluster < d.res_tiles) cluster *= 2;
-    const int blocks = ctx->res_cluster ? cluster : d.res_tiles;
     std::vector<int2> work(blocks);
     for (int b = 0; b < blocks; b++) work[b] = make_int2(0, b);
     auto same = [](const auto &a, const auto &b) {
@@ -2601,6 +2599,18 @@ static int run_resident(ArtContext *ctx, const std::vector<float2> &sched)
                                  ctx->stream));
         ctx->h_sched = sched;
     }
+    return ART_OK;
+}
+
+// The iteration loop of the current solve as one on-chip launch.
+static int run_resident(ArtContext *ctx, const std::vector<float2> &sched)
+{
+    const ImgDev &d = ctx->h_desc[0];
+    int cluster = 1;
+    while (cluster < d.res_tiles) cluster *= 2;
+    const int blocks = ctx->res_cluster ? cluster : d.res_tiles;
+    const int rc = upload_resident(ctx, blocks, sched);
+    if (rc) return rc;
     const size_t smem = res_layout(d).total * sizeof(float);
     const int its = (int)sched.size();
     cudaError_t e;
@@ -2961,6 +2971,47 @@ int32_t art_context_synchronize(ArtContext *ctx)
     ART_CUDA(cudaSetDevice(ctx->device));
     ART_CUDA(cudaStreamSynchronize(ctx->stream));
     return check_errflag(ctx);
+}
+
+int32_t art_context_wait_selftest(ArtContext *ctx, int64_t limit_cycles, int32_t *gave_up)
+{
+    if (!ctx || !gave_up || limit_cycles < 1 || limit_cycles > 8000000000LL)
+        return fail(ART_ERR_INVALID_ARGUMENT, "wait_selftest: bad arguments");
+    ART_CUDA(cudaSetDevice(ctx->device));
+    ctx->net_used = false;
+    const uint32_t W = 2 * RES_TW, H = 160;  // 20 tiles of 16 rows: too many for a cluster
+    float q[64];
+    std::fill(q, q + 64, 1.f);
+    ArtChannel ch{};
+    ch.rounded_px_w = W;
+    ch.rounded_px_h = H;
+    ch.block_w = W / 8;
+    ch.block_h = H / 8;
+    ch.samp_h = ch.samp_v = 1;
+    ch.coef_type = ART_COEF_I16;
+    ch.quant_table = q;
+    int rc;
+    if ((rc = ctx->stage.ensure((size_t)W * H * sizeof(int16_t)))) return rc;
+    ART_CUDA(cudaMemsetAsync(ctx->stage.p, 0, (size_t)W * H * sizeof(int16_t), ctx->stream));
+    const ImageSpec sp{1, &ch, {ctx->stage.p, nullptr, nullptr}, 0.3f, {0.f, 0.f, 0.f}, W, H};
+    const std::vector<float2> sched = iteration_schedule(2, 0, 1.0f, 0.0f);
+    if ((rc = prepare_batch(ctx, {sp}, (uint32_t)sched.size(), ART_INIT_DECODED, 0))) return rc;
+    if (!ctx->resident || ctx->res_cluster)
+        return fail(ART_ERR_UNSUPPORTED, "wait_selftest: the on-chip solver is off or does not fit this GPU");
+    const ImgDev &d = ctx->h_desc[0];
+    const int blocks = d.res_tiles - 1;
+    if ((rc = upload_resident(ctx, blocks, sched))) return rc;
+    const cudaError_t e = launch_resident<1, false>(ctx, blocks, 1, res_layout(d).total * sizeof(float),
+                                                    (int)sched.size(), limit_cycles);
+    const unsigned tag = ctx->res_epoch + 1;
+    ctx->res_epoch += (unsigned)sched.size() + 1;
+    if (e != cudaSuccess) return fail(ART_ERR_CUDA, std::string("wait_selftest: ") + cudaGetErrorString(e));
+    unsigned long long sigma = 0;
+    ART_CUDA(cudaMemcpyAsync(&sigma, d.res_sigma, sizeof(sigma), cudaMemcpyDeviceToHost, ctx->stream));
+    ART_CUDA(cudaStreamSynchronize(ctx->stream));
+    *gave_up = check_errflag(ctx) == ART_ERR_CUDA && (unsigned)(sigma >> 32) != tag;
+    ART_CUDA(cudaMemsetAsync(ctx->errflag, 0, sizeof(unsigned), ctx->stream));
+    return ART_OK;
 }
 
 static int solve_host(ArtContext *ctx, uint32_t nchannel, const ArtChannel *coefs, float weight,

@@ -281,6 +281,17 @@ int32_t art_context_evaluate(ArtContext *ctx, uint32_t image, double out[5]);
 int32_t art_context_synchronize(ArtContext *ctx);
 
 /*
+ * Self-test of the bounded waits of the on-chip solver (the one launch that
+ * solves a small image, its blocks waiting for one another's results): runs a
+ * small solve with one block left out and a limit of limit_cycles clock cycles
+ * (1 .. 8e9) a wait, which a solve sets to about 4e9. The blocks that wait for
+ * the missing one give up, post nothing in its place and return. *gave_up
+ * (host) becomes 1 if they did; a solve would then return ART_ERR_CUDA. The
+ * context stays usable. ART_ERR_UNSUPPORTED where no such solve runs.
+ */
+int32_t art_context_wait_selftest(ArtContext *ctx, int64_t limit_cycles, int32_t *gave_up);
+
+/*
  * Kernel timing of the last device-resident solve on this context, measured
  * with CUDA events around the iteration loop: total milliseconds and, per
  * kernel kind, summed milliseconds over all launches (gradient, update).

@@ -94,3 +94,24 @@ def test_callers_capture_is_refused(gpu, size, sub):
         N.check(call(ctx))
         torch.cuda.synchronize()
     assert all(np.array_equal(o.cpu().numpy().ravel(), w) for o, w in zip(outs, want))
+
+
+def test_waits_give_up(gpu, monkeypatch):
+    """A block that never posts: those that wait for it leave after the limit,
+    nobody is given a step formed without it, and the context solves on."""
+    import time
+
+    monkeypatch.delenv("ART_RESIDENT", raising=False)
+    gave_up = C.c_int32(-1)
+    jpegs = [_jpeg(518, 389, "gray"), _jpeg(200, 136, "4:2:0")]
+    with Context(0) as ctx:
+        want = [_solve(ctx, j) for j in jpegs]
+        for j, w in zip(jpegs, want):
+            t0 = time.perf_counter()
+            N.check(N.lib().art_context_wait_selftest(ctx.handle, 20_000_000, C.byref(gave_up)))
+            assert time.perf_counter() - t0 < 10.0
+            assert gave_up.value == 1
+            N.check(N.lib().art_context_synchronize(ctx.handle))
+            assert _equal(_solve(ctx, j), w)
+        for limit in (0, -1, 8_000_000_001):
+            assert N.lib().art_context_wait_selftest(ctx.handle, limit, C.byref(gave_up)) == N.ART_ERR_INVALID_ARGUMENT
