@@ -157,6 +157,8 @@ EXPORTS = {
                                                 C.POINTER(C.c_uint32)]),
     "art_context_tune_cache": (C.c_int32, [C.c_void_p, C.c_char_p, C.c_int32]),
     "art_context_synchronize": (C.c_int32, [C.c_void_p]),
+    "art_context_set_onchip_limits": (C.c_int32, [C.c_void_p, C.c_int32, C.c_int32]),
+    "art_context_last_onchip": (C.c_int32, [C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "art_context_wait_selftest": (C.c_int32, [C.c_void_p, C.c_int64, C.POINTER(C.c_int32)]),
     "art_context_set_warm_start": (C.c_int32, [C.c_void_p, C.c_void_p]),
     "art_context_set_joint_warm_start": (C.c_int32, [C.c_void_p, C.c_void_p]),

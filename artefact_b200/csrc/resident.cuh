@@ -37,6 +37,7 @@ constexpr int RES_GP = RES_TW + 1;     // row pitch of g: 8x8 blocks of it serve
 constexpr int RES_WARPS = 16;
 constexpr int RES_THREADS = RES_WARPS * 32;
 constexpr int RES_STRIP = 28;          // columns of a norm strip (SWEEP_OUT_N)
+constexpr int RES_CLUSTER = 16;        // blocks of a cluster, at most (a lane each to send a strip's sums to)
 constexpr int RES_CLUSTER_STRIPS = 256;                 // norm strips of an image solved by one cluster, at most
 constexpr int RES_GROUPS = 512;                         // groups of eight norm strips of an image, at most
 constexpr unsigned RES_ERR_TIMEOUT = 2u;                // bit of the solve's error flag

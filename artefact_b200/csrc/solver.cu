@@ -1692,6 +1692,12 @@ struct ImageSpec {
 
 }  // namespace
 
+// What the GPU holds of the on-chip solver: blocks of a cooperative launch, and
+// blocks of the largest cluster (a power of two). Asked once (-1: not yet).
+struct ResLimits {
+    int blocks = -1, cluster = 0;
+};
+
 // Launch shapes of one geometry bucket: gradient-sweep variant (0 narrow, 1
 // wide), strip rows, projection warps per block.
 struct TuneChoice {
@@ -1733,6 +1739,7 @@ struct ArtContext {
     art::DevBuf res_xchg;             // what its blocks exchange (tagged words), and the last tag handed out
     unsigned res_epoch = 0;
     art::DevBuf res_work;
+    art::ResLimits res_limits[4];     // what the GPU holds of k_resident at once, by channel count
     bool timing = false;
     std::vector<cudaEvent_t> events;  // [0,1] loop; then 4 per iteration
     uint32_t timed_iterations = 0;
@@ -2085,6 +2092,43 @@ int multiprocessors(int device)
     return n[device];
 }
 
+// Asks CUDA what it would launch of k_resident with the largest tile. On a part
+// of a GPU (a MIG slice, an MPS share) that is less than on all of it.
+template <int NCH>
+static ResLimits query_resident(int device)
+{
+    ResLimits r;
+    r.blocks = 0;
+    int coop = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_resident<NCH, false>, RES_THREADS, RES_SMEM) == cudaSuccess)
+        r.blocks = per_sm * multiprocessors(device);
+    for (int c = RES_CLUSTER; c > 0 && !r.cluster; c /= 2) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(RES_THREADS);
+        cfg.dynamicSmemBytes = RES_SMEM;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = c;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_resident<NCH, true>, &cfg) == cudaSuccess && n > 0) r.cluster = c;
+    }
+    cudaGetLastError();  // a refusal is an answer
+    return r;
+}
+
+static const ResLimits &resident_limits(ArtContext *ctx, int nch)
+{
+    ResLimits &r = ctx->res_limits[nch];
+    if (r.blocks < 0)
+        r = nch == 3 ? query_resident<3>(ctx->device) : nch == 2 ? query_resident<2>(ctx->device) : query_resident<1>(ctx->device);
+    return r;
+}
+
 // Tiles of one image for the on-chip solver with `rows` rows each: sets the
 // plan in d and returns the tile count, 0 if a tile does not fit a block's
 // shared memory.
@@ -2096,10 +2140,18 @@ static int resident_tiles(ImgDev &d, int rows)
     return d.res_tiles;
 }
 
+// Blocks of the cluster that solves n tiles.
+static int cluster_blocks(int n)
+{
+    int c = 1;
+    while (c < n) c *= 2;
+    return c;
+}
+
 // Chooses between the on-chip solver (k_resident) and the launch pair per
 // iteration. On chip goes one image, solved with the narrow sweep, whose tiles
-// (whole norm strips, a multiple of 16 rows, as few as possible) are all
-// resident at once, at most one a multiprocessor: about 1.3 megapixels of one
+// (whole norm strips, a multiple of 16 rows, as few as possible) the GPU holds
+// all at once, one a multiprocessor: on a whole B200 about 1.3 megapixels of one
 // channel, 0.4 of three. Wherever the tiles fit, it gained: 50 iterations, launch
 // pair -> on chip, 96x64 4:2:0 859 -> 476 us, 518x389 gray 656 -> 388 and 4:4:4
 // 882 -> 683, at the limits 640x480 4:4:4 992 -> 971, 1300x1000 gray 1200 -> 996;
@@ -2121,13 +2173,13 @@ static void plan_resident(ArtContext *ctx)
     if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
     ImgDev &d = ctx->h_desc[0];
     if (d.sweep_kind != 0 || d.nstrips > 8 * RES_GROUPS) return;
-    const int sms = multiprocessors(ctx->device);
+    const ResLimits &lim = resident_limits(ctx, d.nch);
     for (int th = 16; th <= 128 && !ctx->resident; th += 16) {
         if (th % d.strip_rows) continue;
         const int n = resident_tiles(d, th);
         if (!n) break;
-        ctx->resident = n <= sms;
-        ctx->res_cluster = ctx->resident && n <= 16 && d.nstrips <= RES_CLUSTER_STRIPS && env > 1;
+        ctx->res_cluster = n <= RES_CLUSTER && cluster_blocks(n) <= lim.cluster && d.nstrips <= RES_CLUSTER_STRIPS && env > 1;
+        ctx->resident = ctx->res_cluster || n <= lim.blocks;
     }
 }
 
@@ -2602,12 +2654,13 @@ static int upload_resident(ArtContext *ctx, int blocks, const std::vector<float2
     return ART_OK;
 }
 
-// The iteration loop of the current solve as one on-chip launch.
+// The iteration loop of the current solve as one on-chip launch. If CUDA refuses
+// the launch, nothing has run and the solve is no longer one on chip
+// (ctx->resident).
 static int run_resident(ArtContext *ctx, const std::vector<float2> &sched)
 {
     const ImgDev &d = ctx->h_desc[0];
-    int cluster = 1;
-    while (cluster < d.res_tiles) cluster *= 2;
+    const int cluster = cluster_blocks(d.res_tiles);
     const int blocks = ctx->res_cluster ? cluster : d.res_tiles;
     const int rc = upload_resident(ctx, blocks, sched);
     if (rc) return rc;
@@ -2623,7 +2676,10 @@ static int run_resident(ArtContext *ctx, const std::vector<float2> &sched)
             : d.nch == 2 ? launch_resident<2, false>(ctx, blocks, 1, smem, its)
                          : launch_resident<1, false>(ctx, blocks, 1, smem, its);
     ctx->res_epoch += (unsigned)its + 1;
-    if (e != cudaSuccess) return fail(ART_ERR_CUDA, std::string("on-chip solver launch: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // the launch pair meets it again if it was not the launch's own
+        ctx->resident = false;
+    }
     return ART_OK;
 }
 
@@ -2638,7 +2694,8 @@ static int run_iterations(ArtContext *ctx, uint32_t iterations, uint32_t tail = 
     const std::vector<float2> sched = iteration_schedule(iterations, tail, tail_stepmul, decay);
     if (ctx->resident) {
         ctx->timed_iterations = 0;
-        return run_resident(ctx, sched);
+        const int rc = run_resident(ctx, sched);
+        if (rc || ctx->resident) return rc;
     }
     if (ctx->timing) {
         const size_t need = 2 + 4 * (size_t)iterations;
@@ -2971,6 +3028,25 @@ int32_t art_context_synchronize(ArtContext *ctx)
     ART_CUDA(cudaSetDevice(ctx->device));
     ART_CUDA(cudaStreamSynchronize(ctx->stream));
     return check_errflag(ctx);
+}
+
+int32_t art_context_set_onchip_limits(ArtContext *ctx, int32_t blocks, int32_t cluster)
+{
+    if (!ctx || (blocks >= 0 && cluster < 0)) return fail(ART_ERR_INVALID_ARGUMENT, "bad on-chip limits");
+    for (ResLimits &r : ctx->res_limits) {
+        r.blocks = std::max(blocks, -1);
+        r.cluster = blocks < 0 ? 0 : cluster;
+    }
+    return ART_OK;
+}
+
+int32_t art_context_last_onchip(const ArtContext *ctx, int32_t *tiles, int32_t *cluster)
+{
+    if (!ctx || !tiles || !cluster) return fail(ART_ERR_INVALID_ARGUMENT, "null argument");
+    if (ctx->h_desc.empty()) return fail(ART_ERR_INVALID_ARGUMENT, "no solve on this context");
+    *tiles = ctx->resident ? ctx->h_desc[0].res_tiles : 0;
+    *cluster = ctx->resident && ctx->res_cluster;
+    return ART_OK;
 }
 
 int32_t art_context_wait_selftest(ArtContext *ctx, int64_t limit_cycles, int32_t *gave_up)

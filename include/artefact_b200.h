@@ -281,6 +281,18 @@ int32_t art_context_evaluate(ArtContext *ctx, uint32_t image, double out[5]);
 int32_t art_context_synchronize(ArtContext *ctx);
 
 /*
+ * A small image is solved by one launch whose blocks, a tile each, are all on
+ * the GPU at once: a cluster, or a cooperative launch. A context asks CUDA how
+ * many `blocks` of the latter the GPU holds, and how many the largest `cluster`
+ * has; here a caller that shares the GPU says it instead (0 and 0: no such
+ * solves; blocks < 0: ask CUDA). A solve that does not fit, or whose launch CUDA
+ * refuses, runs as two launches per iteration, with the same result.
+ */
+int32_t art_context_set_onchip_limits(ArtContext *ctx, int32_t blocks, int32_t cluster);
+/* Tiles of the last solve if it ran on chip, else 0, and whether as one cluster. */
+int32_t art_context_last_onchip(const ArtContext *ctx, int32_t *tiles, int32_t *cluster);
+
+/*
  * Self-test of the bounded waits of the on-chip solver (the one launch that
  * solves a small image, its blocks waiting for one another's results): runs a
  * small solve with one block left out and a limit of limit_cycles clock cycles
