@@ -1699,9 +1699,10 @@ struct ResLimits {
 };
 
 // Launch shapes of one geometry bucket: gradient-sweep variant (0 narrow, 1
-// wide), strip rows, projection warps per block.
+// wide, 2 quad), strip rows, projection warps per block.
 struct TuneChoice {
     int kind = 0, rows = 0, proj_warps = PROJ_WARPS;
+    bool tuned = false;  // found in the tune cache
 };
 
 }  // namespace art
@@ -1783,14 +1784,25 @@ std::string batch_tune_key(int nimg, long long batch_px)
     return "batch-i" + std::to_string(n) + "-p" + std::to_string(px);
 }
 
+// Launch shapes by size: the narrow sweep unless told otherwise (with its packed
+// channel pair it is the fastest variant from 1080p to 6000x4000 and on the
+// 256-image batch), strips as tall as still give every SM a dozen warps (the 3
+// extra rows a strip reads stay small), and 4 projection warps per block.
+TuneChoice size_shape(long long batch_px, int kind = 0)
+{
+    TuneChoice t;
+    const long long cols = kind == 2 ? SWEEP_OUT_Q : kind == 1 ? SWEEP_OUT : SWEEP_OUT_N;
+    t.kind = kind;
+    t.rows = 128;
+    while (t.rows > 16 && batch_px / (cols * t.rows) < 148LL * 12) t.rows /= 2;
+    return t;
+}
+
 // Launch shapes for one image of a solve of `nimg` images: environment
 // overrides (ART_SWEEP_KIND, ART_STRIP_ROWS, ART_PROJ_WARPS), the candidate
 // the autotuner is timing, the autotuner's choice for the batch's bucket
-// (several images) or the image's bucket (one image), else by size -- the
-// narrow sweep (with its packed channel pair it is the fastest variant from
-// 1080p to 6000x4000 and on the 256-image batch), strips as tall as still
-// give every SM a dozen warps (the 3 extra rows a strip reads stay small), and
-// 4 projection warps per block.
+// (several images) or the image's bucket (one image), else by size
+// (size_shape).
 TuneChoice pick_shape(const ArtContext *ctx, const ImageSpec &sp, long long batch_px, int nimg)
 {
     TuneChoice t;
@@ -1824,13 +1836,11 @@ TuneChoice pick_shape(const ArtContext *ctx, const ImageSpec &sp, long long batc
     }
     if (it != ctx->tune.end()) {
         t = it->second;
+        t.tuned = true;
         if (env_pw_ok) t.proj_warps = env_pw;
         return t;
     }
-    const long long cols = t.kind == 2 ? SWEEP_OUT_Q : t.kind == 1 ? SWEEP_OUT : SWEEP_OUT_N;
-    int R = 128;
-    while (R > 16 && batch_px / (cols * R) < 148LL * 12) R /= 2;
-    t.rows = R;
+    t = size_shape(batch_px, t.kind);
     if (env_pw_ok) t.proj_warps = env_pw;
     return t;
 }
@@ -2162,16 +2172,17 @@ static int cluster_blocks(int n)
 // ART_RESIDENT=0 turns the on-chip solver off, 1 keeps it from forming clusters.
 // A call that the caller's own stream capture has reached gets the launch pair,
 // whose graph launch CUDA refuses there: a replayed on-chip launch would find
-// its own tags in the exchange words and wait for nothing.
-static void plan_resident(ArtContext *ctx)
+// its own tags in the exchange words and wait for nothing. So does the tuner,
+// which chooses between launch pairs, for images of its bucket that do not go
+// on chip.
+static void plan_resident(ArtContext *ctx, ImgDev &d)
 {
     ctx->resident = ctx->res_cluster = false;
     const char *er = getenv("ART_RESIDENT");
     const int env = er ? atoi(er) : 2;
-    if (ctx->h_desc.size() != 1 || ctx->timing || env == 0) return;
+    if (ctx->timing || env == 0 || ctx->strip_rows_override > 0) return;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
-    ImgDev &d = ctx->h_desc[0];
     if (d.sweep_kind != 0 || d.nstrips > 8 * RES_GROUPS) return;
     const ResLimits &lim = resident_limits(ctx, d.nch);
     for (int th = 16; th <= 128 && !ctx->resident; th += 16) {
@@ -2181,6 +2192,19 @@ static void plan_resident(ArtContext *ctx)
         ctx->res_cluster = n <= RES_CLUSTER && cluster_blocks(n) <= lim.cluster && d.nstrips <= RES_CLUSTER_STRIPS && env > 1;
         ctx->resident = ctx->res_cluster || n <= lim.blocks;
     }
+}
+
+// The gradient sweep's strips and blocks of an image.
+static void set_shape(ImgDev &d, const TuneChoice &t)
+{
+    const int out_cols = t.kind == 2 ? SWEEP_OUT_Q : t.kind == 1 ? SWEEP_OUT : SWEEP_OUT_N;
+    const int warps = t.kind == 2 ? SWEEP_WARPS_Q : t.kind == 1 ? SWEEP_WARPS : SWEEP_WARPS_N;
+    d.sweep_kind = t.kind;
+    d.strip_rows = t.rows;
+    d.strips_x = (d.W + out_cols - 1) / out_cols;
+    d.strips_y = (int)(((unsigned)d.H + t.rows - 1) / t.rows);
+    d.nstrips = d.strips_x * d.strips_y;
+    d.ncta = (d.nstrips + warps - 1) / warps;
 }
 
 // Lays out the buffers of a batch of images, uploads descriptors and work
@@ -2207,21 +2231,10 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
         ctx->h_weights[i] = {sp.weight, sp.pweight[0], sp.pweight[1], sp.pweight[2]};
         const int pitch = (int)align_up(sp.W, 32);
         const long long cstride = (long long)pitch * (long long)align_up(sp.H, 32);
-        const TuneChoice sw = pick_shape(ctx, sp, batch_px, nimg);
-        if (i == 0) ctx->proj_warps = sw.proj_warps;
-        const int R = sw.rows;
-        const int out_cols = sw.kind == 2 ? SWEEP_OUT_Q : sw.kind == 1 ? SWEEP_OUT : SWEEP_OUT_N;
-        const int warps = sw.kind == 2 ? SWEEP_WARPS_Q : sw.kind == 1 ? SWEEP_WARPS : SWEEP_WARPS_N;
         d.nch = (int)sp.nch;
         d.W = (int)sp.W;
         d.H = (int)sp.H;
         d.pitch = pitch;
-        d.sweep_kind = sw.kind;
-        d.strip_rows = R;
-        d.strips_x = (int)((sp.W + out_cols - 1) / out_cols);
-        d.strips_y = (int)((sp.H + R - 1) / R);
-        d.nstrips = d.strips_x * d.strips_y;
-        d.ncta = (d.nstrips + warps - 1) / warps;
         d.cstride = cstride;
         // compute_step_tv.rs:130 and compute_step_tv2.rs:88-89, compute_step.rs:47.
         d.alpha_tv = 1.0f / sqrtf((float)sp.nch);
@@ -2231,8 +2244,6 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
         d.step = (sqrtf((float)((uint64_t)sp.W * sp.H)) / 2.0f) / sqrtf(1.0f + (float)step_its);
         o_x[i] = x_floats;
         x_floats += align_up((size_t)3 * sp.nch * cstride, 64);
-        o_misc[i] = misc_bytes;
-        misc_bytes += align_up((size_t)d.ncta * 4 * sizeof(float), 256) + 256;
         for (uint32_t c = 0; c < sp.nch; c++) {
             ChanDev &cd = d.ch[c];
             cd.cw = (int)sp.ch[c].rounded_px_w;
@@ -2255,10 +2266,20 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
                 d.invq2[c][j] = 1.0f / (q * q);
             }
         }
+        const TuneChoice sw = pick_shape(ctx, sp, batch_px, nimg);
+        if (i == 0) ctx->proj_warps = sw.proj_warps;
+        ctx->resident = false;
+        if (nimg == 1) {
+            // A tuned shape is the best launch pair: on chip goes the shape by size.
+            set_shape(d, sw.tuned ? size_shape(batch_px) : sw);
+            plan_resident(ctx, d);
+        }
+        if (!ctx->resident) set_shape(d, sw);
+        o_misc[i] = misc_bytes;
+        misc_bytes += align_up((size_t)d.ncta * 4 * sizeof(float), 256) + 256;
     }
     ctx->l2_fit = l2_fits((x_floats + p_floats) * sizeof(float));
     for (ImgDev &d : ctx->h_desc) d.l2_fit = ctx->l2_fit;
-    plan_resident(ctx);
     if ((rc = ctx->xbuf.ensure(x_floats * sizeof(float)))) return rc;
     if ((rc = ctx->coefimg.ensure(coef_bytes))) return rc;
     if ((rc = ctx->pbuf.ensure(p_floats * sizeof(float)))) return rc;
