@@ -378,13 +378,12 @@ __device__ __forceinline__ void res_sweep_rows(const float *y, int ych, float *g
     }
 }
 
-// work[block] = {image, tile}; sched[k] = {fnext, stepmul} of iteration k, whose
+// One block a tile of the image; sched[k] = {fnext, stepmul} of iteration k, whose
 // tag is epoch + 1 + k. In
 // CLUSTER launches the tiles of one image are one cluster (blocks whose tile
 // index lies past the image's last only keep the barriers complete).
 template <int NCH, bool CLUSTER>
-__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__restrict__ imgs,
-                                                             const int2 *__restrict__ work,
+__global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__restrict__ img,
                                                              const float2 *__restrict__ sched, int iterations,
                                                              unsigned epoch, long long wait_limit, unsigned *err)
 {
@@ -398,19 +397,19 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     __shared__ ImgDev s_im;  // the descriptor, read in every phase
-    const int2 wk = work[blockIdx.x];
+    const int tile = blockIdx.x;
     for (int i = tid; i < (int)(sizeof(ImgDev) / 4); i += RES_THREADS)
-        reinterpret_cast<unsigned *>(&s_im)[i] = __ldg(reinterpret_cast<const unsigned *>(imgs + wk.x) + i);
+        reinterpret_cast<unsigned *>(&s_im)[i] = __ldg(reinterpret_cast<const unsigned *>(img) + i);
     if (tid == 0) s_abort = 0;
     __syncthreads();
     const ImgDev &im = s_im;
     const int ntiles = im.res_tiles;
-    if (CLUSTER && wk.y >= ntiles) {
+    if (CLUSTER && tile >= ntiles) {
         for (int it = 0; it < 2 * iterations; it++) res_cluster_sync();
         return;
     }
     const int W = im.W, H = im.H, pitch = im.pitch, th = im.res_rows, R = im.strip_rows;
-    const int x0 = (wk.y % im.res_tiles_x) * RES_TW, y0 = (wk.y / im.res_tiles_x) * th;
+    const int x0 = (tile % im.res_tiles_x) * RES_TW, y0 = (tile / im.res_tiles_x) * th;
     const ResLayout L = res_layout(im);
     const int ych = (th + 4) * RES_YP, gch = th * RES_GP;
     float *ys = sm + L.y, *gs = sm + L.g;
@@ -456,7 +455,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
     }
     const float at = im.alpha_tv, ag = im.alpha_tgv;
     const float2 nz = make_float2(im.neg_zero, im.neg_zero);
-    const int tcol = wk.y % im.res_tiles_x, trow = wk.y / im.res_tiles_x;
+    const int tcol = tile % im.res_tiles_x, trow = tile / im.res_tiles_x;
     const bool left = tcol > 0, right = tcol + 1 < im.res_tiles_x, up = trow > 0, down = y0 + th < H;
     const int strip0 = (y0 / R) * im.strips_x + x0 / RES_STRIP;  // the tile's first norm strip
     unsigned long long *yx = im.res_y + o0;
@@ -513,7 +512,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
         // polling every strip's words queued their writes behind the polls: with
         // 130 blocks a wait of 5300 to 10000 clocks.)
         if constexpr (CLUSTER) res_cluster_sync();
-        if (CLUSTER || wk.y == 0) {
+        if (CLUSTER || tile == 0) {
             const int n = im.nstrips;
             if constexpr (!CLUSTER) {
                 // 32 neighbouring strips a load; groups of eight added in order.
@@ -603,7 +602,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__res
         if (it + 1 == iterations) break;
         __syncthreads();
         if (ntiles > 1)
-            res_send_border<NCH, CLUSTER>(ys, ych, warp, lane, th, rows, cols, wk.y, im.res_tiles_x, left, right, up, down,
+            res_send_border<NCH, CLUSTER>(ys, ych, warp, lane, th, rows, cols, tile, im.res_tiles_x, left, right, up, down,
                                           yx, cs, pitch, tag);
         if constexpr (CLUSTER) {
             res_cluster_sync();

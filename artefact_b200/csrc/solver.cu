@@ -1734,12 +1734,11 @@ struct ArtContext {
     art::GraphKey key;
     bool resident = false;            // the current solve runs as one on-chip launch (k_resident)
     bool res_cluster = false;         // ... whose blocks form one cluster per image
-    art::DevBuf res_sched;            // its iteration schedule {fnext, stepmul}, and the host copy it holds
-    std::vector<float2> h_sched;
-    std::vector<int2> h_res_work;     // its blocks {image, tile}
-    art::DevBuf res_xchg;             // what its blocks exchange (tagged words), and the last tag handed out
+    std::vector<float2> h_sched;      // its iteration schedule {fnext, stepmul}, as the end of desc holds it
+    // What its blocks exchange (tagged words) lies at the end of xbuf: from which
+    // byte on that holds nothing but such words or zeros, and the last tag used.
+    size_t res_clean = 0;
     unsigned res_epoch = 0;
-    art::DevBuf res_work;
     art::ResLimits res_limits[4];     // what the GPU holds of k_resident at once, by channel count
     bool timing = false;
     std::vector<cudaEvent_t> events;  // [0,1] loop; then 4 per iteration
@@ -2280,26 +2279,43 @@ static int prepare_batch(ArtContext *ctx, const std::vector<ImageSpec> &specs, u
     }
     ctx->l2_fit = l2_fits((x_floats + p_floats) * sizeof(float));
     for (ImgDev &d : ctx->h_desc) d.l2_fit = ctx->l2_fit;
-    if ((rc = ctx->xbuf.ensure(x_floats * sizeof(float)))) return rc;
+    // An on-chip solve takes no buffers of its own: allocating them cost a first
+    // solve 0.5 to 0.8 ms more than the launch pair's (518x389 gray, 20
+    // iterations: 4.4 against 3.8 ms).
+    const size_t x_bytes = align_up(x_floats * sizeof(float), 256);
+    size_t part_bytes = 0, xchg_bytes = 0;
+    if (ctx->resident && !ctx->res_cluster) {
+        const ImgDev &d = ctx->h_desc[0];
+        part_bytes = align_up((size_t)d.nstrips * d.nch * 2 * sizeof(unsigned long long), 256) + 256;
+        xchg_bytes = part_bytes + align_up((size_t)d.nch * d.cstride * sizeof(unsigned long long), 256);
+    }
+    if ((rc = ctx->xbuf.ensure(x_bytes + xchg_bytes))) return rc;
     if ((rc = ctx->coefimg.ensure(coef_bytes))) return rc;
     if ((rc = ctx->pbuf.ensure(p_floats * sizeof(float)))) return rc;
     if ((rc = ctx->misc.ensure(misc_bytes))) return rc;
-    if ((rc = ctx->desc.ensure(nimg * sizeof(ImgDev)))) return rc;
-    if (ctx->resident && !ctx->res_cluster) {
-        // Exchange words of the on-chip solver. Tags only ever grow, so words of
-        // earlier solves never match; new memory, which may hold any word, and a
-        // wrapped count start at zero.
+    const size_t desc_bytes = nimg * sizeof(ImgDev);
+    if ((rc = ctx->desc.ensure(desc_bytes + (ctx->resident ? iterations * sizeof(float2) : 0)))) return rc;
+    if (ctx->desc.fresh || desc_bytes + ctx->h_sched.size() * sizeof(float2) > ctx->desc.n) ctx->h_sched.clear();
+    ctx->desc.fresh = false;
+    // Exchange words of the on-chip solver. Tags only ever grow, so words of
+    // earlier solves never match; new memory, and what planes have covered, may
+    // hold any word and starts at zero, as everything does where the count wraps.
+    if (ctx->xbuf.fresh || (xchg_bytes && ctx->res_epoch > 0xffffffffu - iterations - 2u)) {
+        ctx->xbuf.fresh = false;
+        ctx->res_clean = ctx->xbuf.n;
+        ctx->res_epoch = 0;
+    }
+    ctx->res_clean = std::max(ctx->res_clean, x_bytes);
+    if (xchg_bytes) {
         ImgDev &d = ctx->h_desc[0];
-        const size_t part = align_up((size_t)d.nstrips * d.nch * 2 * sizeof(unsigned long long), 256) + 256;
-        const size_t need = part + (size_t)d.nch * d.cstride * sizeof(unsigned long long);
-        if ((rc = ctx->res_xchg.ensure(need))) return rc;
-        if (ctx->res_xchg.fresh || ctx->res_epoch > 0xffffffffu - iterations - 2u) {
-            ART_CUDA(cudaMemsetAsync(ctx->res_xchg.p, 0, ctx->res_xchg.n, ctx->stream));
-            ctx->res_xchg.fresh = false;
-            ctx->res_epoch = 0;
+        const size_t first = ctx->xbuf.n - xchg_bytes;
+        char *words = static_cast<char *>(ctx->xbuf.p) + first;
+        if (first < ctx->res_clean) {
+            ART_CUDA(cudaMemsetAsync(words, 0, ctx->res_clean - first, ctx->stream));
+            ctx->res_clean = first;
         }
-        d.res_part = static_cast<unsigned long long *>(ctx->res_xchg.p);
-        d.res_y = reinterpret_cast<unsigned long long *>(static_cast<char *>(ctx->res_xchg.p) + part);
+        d.res_part = reinterpret_cast<unsigned long long *>(words);
+        d.res_y = reinterpret_cast<unsigned long long *>(words + part_bytes);
         d.res_sigma = d.res_y - 256 / sizeof(unsigned long long);  // a line of its own between the two
     }
     float *xb = static_cast<float *>(ctx->xbuf.p);
@@ -2624,6 +2640,12 @@ static std::vector<float2> iteration_schedule(uint32_t iterations, uint32_t tail
     return out;
 }
 
+// Place of the schedule h_sched in desc: its end, behind the descriptors.
+static float2 *sched_at(const ArtContext *ctx)
+{
+    return reinterpret_cast<float2 *>(static_cast<char *>(ctx->desc.p) + ctx->desc.n) - ctx->h_sched.size();
+}
+
 template <int NCH, bool CLUSTER>
 static cudaError_t launch_resident(ArtContext *ctx, int blocks, int cluster, size_t smem, int iterations,
                                    long long wait_limit = RES_WAIT_LIMIT)
@@ -2645,32 +2667,19 @@ static cudaError_t launch_resident(ArtContext *ctx, int blocks, int cluster, siz
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_resident<NCH, CLUSTER>, static_cast<const ImgDev *>(ctx->desc.p),
-                              static_cast<const int2 *>(ctx->res_work.p), static_cast<const float2 *>(ctx->res_sched.p),
-                              iterations, ctx->res_epoch, wait_limit, ctx->errflag);
+                              sched_at(ctx), iterations, ctx->res_epoch, wait_limit, ctx->errflag);
 }
 
-// Uploads the blocks {image, tile} and the schedule of an on-chip launch where
-// they are not what the device holds.
-static int upload_resident(ArtContext *ctx, int blocks, const std::vector<float2> &sched)
+// Uploads the schedule of an on-chip launch where it is not what the device holds.
+static int upload_schedule(ArtContext *ctx, const std::vector<float2> &sched)
 {
-    int rc;
-    std::vector<int2> work(blocks);
-    for (int b = 0; b < blocks; b++) work[b] = make_int2(0, b);
-    auto same = [](const auto &a, const auto &b) {
-        return a.size() == b.size() && !memcmp(a.data(), b.data(), a.size() * sizeof(a[0]));
-    };
-    if (!same(work, ctx->h_res_work)) {
-        if ((rc = ctx->res_work.ensure(work.size() * sizeof(int2)))) return rc;
-        ctx->h_res_work.clear();
-        ART_CUDA(cudaMemcpyAsync(ctx->res_work.p, work.data(), work.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
-        ctx->h_res_work = work;
-    }
-    if (!same(sched, ctx->h_sched)) {
-        if ((rc = ctx->res_sched.ensure(sched.size() * sizeof(float2)))) return rc;
+    const size_t bytes = sched.size() * sizeof(float2);
+    if (sched.size() == ctx->h_sched.size() && !memcmp(sched.data(), ctx->h_sched.data(), bytes)) return ART_OK;
+    ctx->h_sched = sched;
+    const cudaError_t e = cudaMemcpyAsync(sched_at(ctx), sched.data(), bytes, cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) {
         ctx->h_sched.clear();
-        ART_CUDA(cudaMemcpyAsync(ctx->res_sched.p, sched.data(), sched.size() * sizeof(float2), cudaMemcpyHostToDevice,
-                                 ctx->stream));
-        ctx->h_sched = sched;
+        return fail(ART_ERR_CUDA, std::string("on-chip schedule: ") + cudaGetErrorString(e));
     }
     return ART_OK;
 }
@@ -2683,7 +2692,7 @@ static int run_resident(ArtContext *ctx, const std::vector<float2> &sched)
     const ImgDev &d = ctx->h_desc[0];
     const int cluster = cluster_blocks(d.res_tiles);
     const int blocks = ctx->res_cluster ? cluster : d.res_tiles;
-    const int rc = upload_resident(ctx, blocks, sched);
+    const int rc = upload_schedule(ctx, sched);
     if (rc) return rc;
     const size_t smem = res_layout(d).total * sizeof(float);
     const int its = (int)sched.size();
@@ -2876,9 +2885,6 @@ void art_context_destroy(ArtContext *ctx)
     ctx->sepplanes.release();
     ctx->rgb.release();
     ctx->pred.release();
-    ctx->res_sched.release();
-    ctx->res_work.release();
-    ctx->res_xchg.release();
     ctx->evalbuf.release();
     ctx->hstage.release();
     ctx->hrgb.release();
@@ -3097,7 +3103,7 @@ int32_t art_context_wait_selftest(ArtContext *ctx, int64_t limit_cycles, int32_t
         return fail(ART_ERR_UNSUPPORTED, "wait_selftest: the on-chip solver is off or does not fit this GPU");
     const ImgDev &d = ctx->h_desc[0];
     const int blocks = d.res_tiles - 1;
-    if ((rc = upload_resident(ctx, blocks, sched))) return rc;
+    if ((rc = upload_schedule(ctx, sched))) return rc;
     const cudaError_t e = launch_resident<1, false>(ctx, blocks, 1, res_layout(d).total * sizeof(float),
                                                     (int)sched.size(), limit_cycles);
     const unsigned tag = ctx->res_epoch + 1;

@@ -115,3 +115,38 @@ def test_waits_give_up(gpu, monkeypatch):
             assert _equal(_solve(ctx, j), w)
         for limit in (0, -1, 8_000_000_001):
             assert N.lib().art_context_wait_selftest(ctx.handle, limit, C.byref(gave_up)) == N.ART_ERR_INVALID_ARGUMENT
+
+
+@pytest.mark.parametrize("size,sub,words", [((96, 64), "4:2:0", 0), ((518, 389), "gray", 2)])
+def test_no_buffers_of_its_own(gpu, monkeypatch, size, sub, words):
+    """A first solve allocates what the launch pair's does, and room in the same
+    buffers for the exchange words (MiB)."""
+    import torch
+
+    j = _jpeg(*size, sub)
+    taken = {}
+    for mode in ("0", "2"):
+        monkeypatch.setenv("ART_RESIDENT", mode)
+        taken[mode] = []
+        for _ in range(4):  # the first solve of a process also sets CUDA up
+            with Context(0) as ctx:
+                before = torch.cuda.mem_get_info()[0]
+                _solve(ctx, j)
+                taken[mode].append((before - torch.cuda.mem_get_info()[0]) >> 20)
+    assert min(taken["2"]) <= min(taken["0"]) + words, taken
+
+
+def test_planes_over_exchange_words(gpu, monkeypatch):
+    """Planes of a larger solve cover the place of earlier exchange words."""
+    small, large = _jpeg(518, 389, "gray"), _jpeg(720, 600, "gray")
+    monkeypatch.setenv("ART_RESIDENT", "0")
+    with Context(0) as ctx:
+        want = [_solve(ctx, small), _solve(ctx, large)]
+    with Context(0) as ctx:
+        for _ in range(2):
+            monkeypatch.setenv("ART_RESIDENT", "2")
+            assert _equal(_solve(ctx, small), want[0])
+            monkeypatch.setenv("ART_RESIDENT", "0")
+            assert _equal(_solve(ctx, large), want[1])
+            monkeypatch.setenv("ART_RESIDENT", "2")
+            assert _equal(_solve(ctx, large), want[1])
