@@ -554,25 +554,33 @@ __global__ void __launch_bounds__(THREADS, 1) k_wgrad3x3(const __grid_constant__
 }
 
 // dW[n][tap][c] (+)= sum over bands of the partials. Bound by latency (a few MB
-// in all): a block takes 32 neighbouring partials, each of its eight warps an
-// eighth of the bands, and adds the warps' sums in order. One thread an output
-// took 11 to 27 us with up to 256 bands.
+// in all): with SPLIT = 8 a block takes 32 neighbouring partials, each of its
+// eight warps an eighth of the bands, and adds the warps' sums in order. One
+// thread an output took 11 to 27 us with up to 256 bands. Up to eight bands
+// SPLIT = 1 does that all the same: the sums are the same ones, and splitting
+// them leaves warps without a band (2 bands, 512 to 128 channels of 7x33 pixels,
+// with k_wgrad3x3 before it: 33.6 us split, 23.6 not).
+template <int SPLIT>
 __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ partial, int bands, int cout, int cin,
                                                       int nci, float *__restrict__ dw, int accumulate)
 {
-    __shared__ float s[8][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int N = 256 / SPLIT;  // partials of a block
+    const int k = threadIdx.x / N, i = threadIdx.x % N;
     const int total = cout * 9 * cin;  // a multiple of 32
-    const int e = blockIdx.x * 32 + lane;  // index of a band's partials [chunk][tap][n][cc]
+    const int e = blockIdx.x * N + i;  // index of a band's partials [chunk][tap][n][cc]
     float t = 0.f;
+    if (SPLIT == 1 && e >= total) return;
 #pragma unroll 8
-    for (int b = warp; b < bands; b += 8) t += partial[(size_t)b * total + e];
-    s[warp][lane] = t;
-    __syncthreads();
-    if (warp) return;
-    t = s[0][lane];
+    for (int b = k; b < bands; b += SPLIT) t += partial[(size_t)b * total + e];
+    if constexpr (SPLIT > 1) {
+        __shared__ float s[SPLIT][N];
+        s[k][i] = t;
+        __syncthreads();
+        if (k) return;
+        t = s[0][i];
 #pragma unroll
-    for (int w = 1; w < 8; w++) t += s[w][lane];
+        for (int w = 1; w < SPLIT; w++) t += s[w][i];
+    }
     const int cc = e % nci, n = e / nci % cout, tap = e / (nci * cout) % 9, chunk = e / (nci * cout * 9);
     float *o = dw + ((size_t)n * 9 + tap) * cin + chunk * nci + cc;
     *o = accumulate ? *o + t : t;
@@ -1571,7 +1579,9 @@ int32_t wgrad3x3(const ArtCnnWgrad *d, cudaStream_t s)
     int32_t rc = check_launch("k_wgrad3x3");
     if (rc) return rc;
     const int total = d->cout * 9 * d->cin;
-    k_wgrad_reduce<<<total / 32, 256, 0, s>>>(a.partial, bands, d->cout, d->cin, nci, d->dw, d->accumulate);
+    const auto reduce = bands > 8 ? k_wgrad_reduce<8> : k_wgrad_reduce<1>;
+    reduce<<<bands > 8 ? total / 32 : (total + 255) / 256, 256, 0, s>>>(a.partial, bands, d->cout, d->cin, nci, d->dw,
+                                                                        d->accumulate);
     return check_launch("k_wgrad_reduce");
 }
 
