@@ -1608,7 +1608,16 @@ int32_t colsum_partial(const bf16 *g, long long npix, int C, int nblk, float *pa
 
 int32_t colsum_final(const ColsumList &list, cudaStream_t s)
 {
-    k_colsum_final<<<list.count, 1024, 0, s>>>(list);
+    // A thread takes four partials of a channel or more, and a channel 64 threads
+    // at most, since one of them adds their sums: with all 1024 for one channel
+    // that alone took 4 us (one pixel, one channel: 13.6 us, now 11.3).
+    int threads = 32;
+    for (int i = 0; i < list.count; i++) {
+        const ColsumItem &it = list.item[i];
+        threads = std::max(threads, it.C * std::min((it.nblk + 3) / 4, 64));
+    }
+    threads = std::min((threads + 31) / 32 * 32, 1024);
+    k_colsum_final<<<list.count, threads, 0, s>>>(list);
     return check_launch("k_colsum_final");
 }
 

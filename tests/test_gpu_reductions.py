@@ -40,3 +40,21 @@ def test_weight_gradient_bands(gpu, bands, cin, cout, accumulate):
     ref = O.conv_wgrad(x, g) + 0.5 * accumulate
     np.testing.assert_allclose(got[:total].reshape(cout, 9, cin), ref, rtol=0, atol=2e-5 * float(np.abs(ref).max()) + 1e-5)
     assert (got[total:] == 0.5).all()
+
+
+@pytest.mark.parametrize("blocks", [1, 4, 5, 17, 257])
+@pytest.mark.parametrize("channels", [1, 2, 16, 33, 256])
+def test_bias_gradient_partials(gpu, blocks, channels):
+    """The workspace sets the number of partials. fp32 sums of at most 4001 terms
+    in a row: an error of 4096 units of 2^-24 of the sum of magnitudes bounds any
+    order."""
+    import torch
+    npix = 4001
+    g = torch.randn(npix * channels, device="cuda", generator=torch.Generator("cuda").manual_seed(blocks)).to(torch.bfloat16)
+    ws = torch.empty(blocks * channels * 4, dtype=torch.uint8, device="cuda")
+    out = torch.full((channels,), 2.0, device="cuda")
+    N.check(N.lib().art_cnn_bias_grad(g.data_ptr(), npix, channels, ws.data_ptr(), ws.numel(), out.data_ptr(), 1, None))
+    torch.cuda.synchronize()
+    g64 = g.double().reshape(npix, channels)
+    bound = 4096 * 2.0**-24 * (g64.abs().sum(0) + 2)
+    assert bool(((out.double() - g64.sum(0) - 2).abs() <= bound).all())
