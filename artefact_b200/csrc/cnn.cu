@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ 
 // Forward: n = output channel, k = input channel. Transposed (backward-data):
 // n = input channel ci0 + n, k = output channel, taps mirrored.
 // A launch packs every layer of a list; a thread makes one 16-byte piece. The
-// weights are few (1 MB): a launch a pack took 23 x 3.3 us of a training step.
+// weights are few (1 MB): a launch a pack took 18 x 3.5 us of a training step.
 struct PackItem {
     const float *w;
     bf16 *out;

@@ -379,9 +379,8 @@ __device__ __forceinline__ void res_sweep_rows(const float *y, int ych, float *g
 }
 
 // One block a tile of the image; sched[k] = {fnext, stepmul} of iteration k, whose
-// tag is epoch + 1 + k. In
-// CLUSTER launches the tiles of one image are one cluster (blocks whose tile
-// index lies past the image's last only keep the barriers complete).
+// tag is epoch + 1 + k. In CLUSTER launches the tiles are one cluster (blocks
+// whose index lies past the last tile only keep the barriers complete).
 template <int NCH, bool CLUSTER>
 __global__ void __launch_bounds__(RES_THREADS, 1) k_resident(const ImgDev *__restrict__ img,
                                                              const float2 *__restrict__ sched, int iterations,

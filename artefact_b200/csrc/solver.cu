@@ -513,7 +513,7 @@ __device__ __forceinline__ void narrow_row(NarrowGroup<float> &A, NarrowGroup<fl
 // the walk wait (a warp has six scoreboards for all its loads, shuffles and
 // special functions, so waiting for a shuffle could mean waiting for the newest
 // global load), and a third of its 215 instructions per row of 32 columns were
-// addresses, clamps and moves; now it issues 196, 92 of them arithmetic, at 65 %
+// addresses, clamps and moves; now it issues 196, 92 of them arithmetic, at 63 %
 // of the issue slots, which with the tail below bounds it. Measured per launch,
 // before -> now: 1920x1080 4:4:4 33.9 -> 31.1 us, 2600x1500 4:4:4 55.8 -> 49.1,
 // 4:2:0 52.9 -> 48.5, 200x136 gray 13.8 -> 11.7. Two columns a lane halve the
